@@ -461,20 +461,14 @@ kate_status kate_sim_destroy(kate_sim* s) {
 kate_status kate_sim_execute(kate_sim* s, double* theta_phi) {
     return guarded([&] {
         REQUIRE(s, "null simulator");
-        std::string e = s->sim->run_async(nullptr, nullptr);
-        if (e.empty()) e = s->sim->synchronize();
-        if (e.empty() && theta_phi) e = s->sim->proba_state(theta_phi);
-        return sim_status(e);
+        return sim_status(s->sim->execute(nullptr, theta_phi));
     });
 }
 
 kate_status kate_sim_execute_from(kate_sim* s, const double* in, double* out) {
     return guarded([&] {
         REQUIRE(s && in, "null pointer");
-        std::string e = s->sim->run_async(nullptr, in);
-        if (e.empty()) e = s->sim->synchronize();
-        if (e.empty() && out) e = s->sim->proba_state(out);
-        return sim_status(e);
+        return sim_status(s->sim->execute(in, out));
     });
 }
 

@@ -3,6 +3,7 @@
 
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 namespace kate {
 
@@ -17,6 +18,8 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 Block g_cached[kMaxDevices];                   // one released buffer per device
 std::unordered_map<void*, size_t> g_live;      // buffers handed out, with their real size
+char* g_slab = nullptr;                        // pinned slots
+std::vector<char*> g_free_slots;
 
 void free_cached_locked(int device) {
     Block& c = g_cached[device];
@@ -76,6 +79,34 @@ void release_cached(int device) {
         return;
     }
     for (int d = 0; d < kMaxDevices; d++) free_cached_locked(d);
+    if (g_slab && (int)g_free_slots.size() == kPinnedSlots) {
+        cudaFreeHost(g_slab);
+        g_slab = nullptr;
+        g_free_slots.clear();
+    }
+}
+
+void* pinned_take() {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_slab) {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kPinnedSlotBytes * kPinnedSlots, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        g_slab = static_cast<char*>(p);
+        for (int i = kPinnedSlots; i-- > 0;) g_free_slots.push_back(g_slab + (size_t)i * kPinnedSlotBytes);
+    }
+    if (g_free_slots.empty()) return nullptr;
+    void* p = g_free_slots.back();
+    g_free_slots.pop_back();
+    return p;
+}
+
+void pinned_give(void* p) {
+    if (!p) return;
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_free_slots.push_back(static_cast<char*>(p));
 }
 
 }  // namespace kate

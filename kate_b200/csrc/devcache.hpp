@@ -26,7 +26,19 @@ cudaError_t cached_malloc(void** p, size_t bytes, int device);
 // Releases a buffer from cached_malloc (the current device is `device`).
 // Waits for the device first, so no kernel still uses it when it is reused.
 void cached_free(void* p, int device);
-// Frees the cached buffer of `device` (-1: of every device).
+// Frees the cached buffer of `device` (-1: of every device) and, for -1, the
+// pinned slab below when none of its slots is out.
 void release_cached(int device);
+
+// Pinned host memory for small results (a measurement's sums, samples): slots
+// of kPinnedSlotBytes from one slab of kPinnedSlots, allocated at the first
+// request and mapped into every device's address space, so that a kernel
+// writes its results where the host reads them. pinned_take returns null when
+// no slot (or no pinned memory) is left; the caller then copies from device
+// memory. A slot belongs to its taker until pinned_give. Thread-safe.
+constexpr size_t kPinnedSlotBytes = 16 * 1024;
+constexpr int kPinnedSlots = 64;
+void* pinned_take();
+void pinned_give(void* p);
 
 }  // namespace kate

@@ -4,13 +4,22 @@
 // amplitudes whose bit b is 0 and the sum over those whose bit b is 1 (kind
 // 0: the amplitudes themselves, the reference's proba_state input,
 // HIPcode/simulator.hpp:40-61 and 483-543; kind 1: |a|^2, for <Z_q>), in one
-// read pass. Element x is split as
-//   x = ((r << g) | cta) << 12 | j << 8 | t
-// (t = thread, j = 0..15 unrolled, cta = blockIdx, r = round). The sums over
-// t-bits and j-bits are exact subset sums of per-thread accumulators; the
-// cta-bits are resolved on the host from per-CTA totals; r-bits are
-// accumulated per thread. Each CTA writes its partials; the host adds them
-// in CTA order (deterministic).
+// read pass; k_bitsums_finish adds the CTAs' partials on the device, so the
+// host receives 2n + 1 sums. Amplitude x is split as
+//   x = ((r << g) | cta) << 12 | (12 local bits)
+// and every 16-byte load of a thread covers one complex128 amplitude (local
+// bits 0..7 = thread, 8..11 = load) or two complex64 ones (bit 0 = within
+// the load, 1..8 = thread, 9..11 = load): 16 amplitudes per thread and
+// round. Bits held inside a thread are summed by a tree over the 16 values
+// (2.75 additions per amplitude where one running sum per bit takes 5),
+// thread bits once per CTA, round bits from per-round warp totals kept in
+// shared memory, CTA bits by the finishing kernel. Every order is fixed by
+// the shape, so results repeat.
+//
+// Bound by HBM: the state is read once. Loads are issued eight at a time
+// into registers before they are added; with one running sum per bit and
+// per round bit in registers the amplitude form held 128 registers and read
+// 1 GiB in 416 us (2.6 TB/s).
 #include "k_common.cuh"
 #include "launch.hpp"
 
@@ -40,105 +49,174 @@ struct Acc<double> {
     __device__ static double shfl(double v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
 };
 
-// Output slots per CTA: 0 = total; 1 + 2*b = bit b is 0; 2 + 2*b = bit b is
-// 1, for local bits b = 0..11 then round bits 12..12+nr-1 (numbered in slot
-// order, not in index order).
 __device__ __forceinline__ double2 ld_amp(const double2* p) { return *p; }
 __device__ __forceinline__ double2 ld_amp(const float2* p) {
     const float2 v = *p;
     return make_double2(v.x, v.y);
 }
 
-// S: stored amplitude type (double2 or float2); sums are FP64 either way.
-template <typename V, typename S = double2>
-__global__ void __launch_bounds__(NT, 2) k_bitsums(const S* __restrict__ st, int n, int g, int nr,
-                                                V* __restrict__ part) {
+// Half a thread's round (8 amplitudes, in-thread bits 0..2 of their index)
+// at element x0 of the round: values of element x >= lim are zero. With
+// SCALE the amplitudes are first multiplied by f (one rounding) and stored.
+template <typename V, bool SCALE>
+__device__ __forceinline__ void load_half(const double2* st, uint32_t t, uint32_t h, uint32_t lim, double, V (&v)[8]) {
+    static_assert(!SCALE, "complex128 states are not rescaled");
+    double2 a[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint32_t x = t + ((h * 8u + (uint32_t)k) << 8);
+        a[k] = x < lim ? __ldcs(st + x) : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = Acc<V>::val(a[k]);
+}
+template <typename V, bool SCALE>
+__device__ __forceinline__ void load_half(float2* st, uint32_t t, uint32_t h, uint32_t lim, double f, V (&v)[8]) {
+    float4 a[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint32_t x = 2u * t + ((h * 4u + (uint32_t)k) << 9);
+        a[k] = x < lim ? __ldcs(reinterpret_cast<const float4*>(st + x)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    if constexpr (SCALE) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            a[k].x = (float)((double)a[k].x * f);
+            a[k].y = (float)((double)a[k].y * f);
+            a[k].z = (float)((double)a[k].z * f);
+            a[k].w = (float)((double)a[k].w * f);
+            const uint32_t x = 2u * t + ((h * 4u + (uint32_t)k) << 9);
+            if (x < lim) __stcs(reinterpret_cast<float4*>(st + x), a[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[2 * k] = Acc<V>::val(make_double2(a[k].x, a[k].y));
+        v[2 * k + 1] = Acc<V>::val(make_double2(a[k].z, a[k].w));
+    }
+}
+
+// Partials of CTA c, slot i: part[i * gridDim.x + c]. Slot 0 is the total,
+// 1 + 2b / 2 + 2b the sums with bit b 0 / 1, for the local bits b = 0..11,
+// then the round bits 12..12+nr-1 (in slot order, not index order). With
+// one CTA and no rounds that is k_bitsums_finish's output already.
+// SCALE (complex64): every amplitude is also multiplied by scale[1] and
+// written back (the renormalisation, whose pass over the state this saves).
+template <typename V, typename S, bool SCALE = false>
+__global__ void __launch_bounds__(NT, 3) k_bitsums(S* __restrict__ st, int n, int g, int nr, V* __restrict__ part,
+                                                   const double* __restrict__ scale, const int* __restrict__ err,
+                                                   int* __restrict__ err_out) {
     using A = Acc<V>;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int lb = n < 12 ? n : 12;
-    const uint32_t lim = 1u << lb;
-    V T = A::zero(), H0[4], H1[4], R0[MAXR], R1[MAXR];
+    if (err_out && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
+    constexpr bool F = sizeof(S) == 8;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    const uint32_t lim = 1u << (n < 12 ? n : 12);
+    const uint32_t rounds = 1u << nr;
+    extern __shared__ __align__(16) unsigned char bs_raw[];
+    V* rtot = reinterpret_cast<V*>(bs_raw);  // [rounds][8] warp totals (nr > 0)
+    __shared__ V st_t[NT];
+    __shared__ V sw[NT / 32][8];
+    double f = 1.0;
+    if constexpr (SCALE) f = scale[1];
+    // H[2i] / H[2i + 1]: in-thread bit i is 0 / 1.
+    V H[8];
 #pragma unroll
-    for (int i = 0; i < 4; i++) H0[i] = H1[i] = A::zero();
-#pragma unroll
-    for (int i = 0; i < MAXR; i++) R0[i] = R1[i] = A::zero();
-    const uint64_t rounds = 1ull << nr;
-    for (uint64_t r = 0; r < rounds; r++) {
-        const uint64_t base = ((r << g) | blockIdx.x) << 12;
+    for (int i = 0; i < 8; i++) H[i] = A::zero();
+    for (uint32_t r = 0; r < rounds; r++) {
+        S* base = st + ((((uint64_t)r << g) | blockIdx.x) << 12);
         V tr = A::zero();
 #pragma unroll
-        for (int j = 0; j < 16; j++) {
-            const uint32_t x = (uint32_t)t + ((uint32_t)j << 8);
-            V v = A::zero();
-            if (x < lim) v = A::val(ld_amp(st + base + x));
-            tr = A::add(tr, v);
+        for (uint32_t h = 0; h < 2; h++) {
+            V v[8], p[4];
+            load_half<V, SCALE>(base, t, h, lim, f, v);
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                if ((j >> i) & 1) H1[i] = A::add(H1[i], v);
-                else H0[i] = A::add(H0[i], v);
-            }
+            for (int k = 0; k < 4; k++) p[k] = A::add(v[2 * k], v[2 * k + 1]);
+            H[0] = A::add(H[0], A::add(A::add(v[0], v[2]), A::add(v[4], v[6])));
+            H[1] = A::add(H[1], A::add(A::add(v[1], v[3]), A::add(v[5], v[7])));
+            const V q0 = A::add(p[0], p[1]), q1 = A::add(p[2], p[3]);
+            H[2] = A::add(H[2], A::add(p[0], p[2]));
+            H[3] = A::add(H[3], A::add(p[1], p[3]));
+            H[4] = A::add(H[4], q0);
+            H[5] = A::add(H[5], q1);
+            const V s = A::add(q0, q1);
+            H[6 + h] = A::add(H[6 + h], s);
+            tr = A::add(tr, s);
         }
-        T = A::add(T, tr);
+        if (nr) {
 #pragma unroll
-        for (int i = 0; i < MAXR; i++)
-            if (i < nr) {
-                if ((r >> i) & 1) R1[i] = A::add(R1[i], tr);
-                else R0[i] = A::add(R0[i], tr);
-            }
-    }
-    // Slots reduced per warp: 0 total; 1..5 lane-bit-1 sums; 6..10
-    // lane-bit-0 sums; 11..14 H0; 15..18 H1; 19.. R0; 19+MAXR.. R1.
-    constexpr int NS = 19 + 2 * MAXR;
-    __shared__ V sm[NT / 32][NS];
-    auto wsum = [&](V v) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v = A::add(v, A::shfl(v, o));
-        return v;
-    };
-    V w;
-    w = wsum(T);
-    if (lane == 0) sm[warp][0] = w;
-#pragma unroll
-    for (int b = 0; b < 5; b++) {
-        w = wsum(((lane >> b) & 1) ? T : A::zero());
-        if (lane == 0) sm[warp][1 + b] = w;
-        w = wsum(((lane >> b) & 1) ? A::zero() : T);
-        if (lane == 0) sm[warp][6 + b] = w;
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        w = wsum(H0[i]);
-        if (lane == 0) sm[warp][11 + i] = w;
-        w = wsum(H1[i]);
-        if (lane == 0) sm[warp][15 + i] = w;
-    }
-#pragma unroll
-    for (int i = 0; i < MAXR; i++) {
-        if (i < nr) {
-            w = wsum(R0[i]);
-            if (lane == 0) sm[warp][19 + i] = w;
-            w = wsum(R1[i]);
-            if (lane == 0) sm[warp][19 + MAXR + i] = w;
+            for (int o = 16; o > 0; o >>= 1) tr = A::add(tr, A::shfl(tr, o));
+            if (lane == 0) rtot[r * (NT / 32) + warp] = tr;
         }
+    }
+    st_t[t] = A::add(H[6], H[7]);
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        V w = H[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) w = A::add(w, A::shfl(w, o));
+        if (lane == 0) sw[warp][i] = w;
     }
     __syncthreads();
-    const int nout = 1 + 2 * (12 + nr);
-    if (t < nout) {
+    const uint32_t ncta = gridDim.x, c = blockIdx.x;
+    {
+        // Thread bits: 16 threads per (bit, value), 8 of the 128 threads'
+        // totals each.
+        const uint32_t b = t >> 5, one = (t >> 4) & 1u, i = t & 15u;
         V s = A::zero();
-        if (t == 0) {
-            for (int ww = 0; ww < NT / 32; ww++) s = A::add(s, sm[ww][0]);
-        } else {
-            const int b = (t - 1) / 2, one = (t - 1) & 1;
-            for (int ww = 0; ww < NT / 32; ww++) {
-                V v;
-                if (b < 5) v = one ? sm[ww][1 + b] : sm[ww][6 + b];
-                else if (b < 8) v = (((ww >> (b - 5)) & 1) == one) ? sm[ww][0] : A::zero();
-                else if (b < 12) v = one ? sm[ww][15 + (b - 8)] : sm[ww][11 + (b - 8)];
-                else v = one ? sm[ww][19 + MAXR + (b - 12)] : sm[ww][19 + (b - 12)];
-                s = A::add(s, v);
-            }
-        }
-        part[(size_t)blockIdx.x * nout + t] = s;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) s = A::add(s, st_t[ins0(i + 16u * k, (int)b) | (one << b)]);
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) s = A::add(s, A::shfl(s, o));
+        const uint32_t bit = F ? b + 1u : b;
+        if (i == 0) part[(size_t)(1 + 2 * bit + one) * ncta + c] = s;
+        // The total: the two halves of thread bit 0.
+        const V other = A::shfl(s, 16);
+        if (t == 0) part[c] = A::add(s, other);
+    }
+    if (t < 8) {
+        V s = A::zero();
+#pragma unroll
+        for (int w = 0; w < NT / 32; w++) s = A::add(s, sw[w][t]);
+        const uint32_t i = t >> 1, bit = F ? (i == 0 ? 0u : 8u + i) : 8u + i;
+        part[(size_t)(1 + 2 * bit + (t & 1u)) * ncta + c] = s;
+    }
+    if (t >= 32 && t < 32 + 2u * (uint32_t)nr) {
+        const uint32_t i = (t - 32u) >> 1, one = t & 1u;
+        V s = A::zero();
+        for (uint32_t r = 0; r < rounds; r++)
+            if (((r >> i) & 1u) == one)
+                for (int w = 0; w < NT / 32; w++) s = A::add(s, rtot[r * (NT / 32) + w]);
+        part[(size_t)(1 + 2 * (12 + i) + one) * ncta + c] = s;
+    }
+}
+
+// One CTA per output, from output `first`: out[0] = total, out[1 + 2b + v] =
+// sum over the amplitudes whose index bit b is v. Partials are added per
+// thread in CTA order, then in a fixed tree.
+template <typename V>
+__global__ void __launch_bounds__(NT) k_bitsums_finish(const V* __restrict__ part, int g, int first,
+                                                       V* __restrict__ out) {
+    using A = Acc<V>;
+    const uint32_t o = blockIdx.x + (uint32_t)first, t = threadIdx.x, ncta = 1u << g;
+    const int b = o ? (int)(o - 1) / 2 : 0, one = o ? (int)(o - 1) & 1 : 0;
+    const bool cta_bit = o && b >= 12 && b < 12 + g;
+    int slot = 0;  // the totals, for o = 0 and for CTA bits
+    if (o && b < 12) slot = (int)o;
+    else if (o && !cta_bit) slot = 1 + 2 * (b - g) + one;
+    const V* p = part + (size_t)slot * ncta;
+    V s = A::zero();
+    for (uint32_t c = t; c < ncta; c += NT)
+        if (!cta_bit || (int)((c >> (b - 12)) & 1u) == one) s = A::add(s, p[c]);
+    __shared__ V red[NT / 32];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s = A::add(s, A::shfl(s, d));
+    if ((t & 31u) == 0) red[t >> 5] = s;
+    __syncthreads();
+    if (t == 0) {
+        s = red[0];
+#pragma unroll
+        for (int w = 1; w < NT / 32; w++) s = A::add(s, red[w]);
+        out[o] = s;
     }
 }
 
@@ -154,7 +232,7 @@ __global__ void k_probs(const S* __restrict__ st, uint64_t dim, double* __restri
 // ||psi||^2 in FP64: each CTA sums |a|^2 over a grid-stride range (16-byte
 // loads, two amplitudes each, in a fixed per-thread order), reduces it in a
 // fixed tree, writes its partial; the last CTA to finish adds the partials
-// in CTA order (deterministic) and writes out[0] = ||psi||^2 and out[1] =
+// in a fixed order (deterministic) and writes out[0] = ||psi||^2 and out[1] =
 // 1 / ||psi||, then resets the counter for the next run.
 constexpr int RN_GRID = 148 * 4;
 
@@ -191,10 +269,20 @@ __global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st
         last = atomicAdd(count, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && t == 0) {
-        __threadfence();
-        double tot = 0.0;
-        for (uint32_t c = 0; c < gridDim.x; c++) tot += ((volatile double*)part)[c];
+    if (!last) return;
+    // Partials by the whole CTA, in a fixed order (one thread adding 592 of
+    // them one after another took 20 us, most of the kernel at 21 qubits).
+    __threadfence();
+    double tot = 0.0;
+    for (uint32_t c = t; c < gridDim.x; c += 256) tot += __ldcg(part + c);
+    red[t] = tot;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+        if (t < (uint32_t)w) red[t] += red[t + w];
+        __syncthreads();
+    }
+    if (t == 0) {
+        tot = red[0];
         out[0] = tot;
         out[1] = tot > 0.0 ? 1.0 / sqrt(tot) : 1.0;
         *count = 0;
@@ -224,7 +312,7 @@ __global__ void __launch_bounds__(256) k_scale_c64(float4* __restrict__ st, uint
 
 size_t renorm_scratch_bytes() { return (RN_GRID + 4) * sizeof(double); }
 
-cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
+cudaError_t launch_norm_c64(const void* st, int n, void* scratch, cudaStream_t s) {
     if (n < 1) return cudaErrorInvalidValue;
     const uint64_t npairs = (1ull << n) / 2;
     double* part = (double*)scratch;
@@ -232,71 +320,85 @@ cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
     unsigned* count = (unsigned*)(out + 2);
     const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
     k_norm2_c64<<<grid, 256, 0, s>>>((const float4*)st, npairs, part, count, out);
-    cudaError_t e = cudaGetLastError();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
+    const cudaError_t e = launch_norm_c64(st, n, scratch, s);
     if (e != cudaSuccess) return e;
-    k_scale_c64<<<grid, 256, 0, s>>>((float4*)st, npairs, out);
+    const uint64_t npairs = (1ull << n) / 2;
+    const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
+    k_scale_c64<<<grid, 256, 0, s>>>((float4*)st, npairs, (const double*)scratch + RN_GRID);
     return cudaGetLastError();
 }
 
 BitSumShape bitsum_shape(int n) {
     BitSumShape s{};
-    if (n <= 12) {
-        s.g = 0;
-        s.nr = 0;
-    } else {
-        // About a thousand CTAs (seven per SM), each summing up to 2^MAXR
-        // rounds in registers: few partials to add on the host.
-        s.g = n - 12 < 10 ? n - 12 : 10;
-        s.nr = n - 12 - s.g;
-        if (s.nr > MAXR) {
-            s.nr = MAXR;
-            s.g = n - 12 - MAXR;
-        }
+    if (n > 12) {
+        // One CTA per tile up to 22 qubits (latency: every SM busy), then up
+        // to 16 rounds per CTA, which keeps the partials under 1/1000 of the
+        // state and leaves thousands of CTAs (2^14 at 30 qubits: 37 waves of
+        // 3 per SM, so a last partial wave costs nothing).
+        s.nr = n > 30 ? n - 26 : n > 26 ? 4 : n > 22 ? n - 22 : 0;
+        if (s.nr > MAXR) s.nr = MAXR;
+        s.g = n - 12 - s.nr;
     }
     s.grid = 1 << s.g;
     s.nout = 1 + 2 * (12 + s.nr);
     return s;
 }
 
-cudaError_t launch_bitsums_c128(const void* st, int n, int kind, void* partials, cudaStream_t s) {
-    BitSumShape sh = bitsum_shape(n);
-    if (sh.nr > MAXR) return cudaErrorInvalidValue;
-    if (kind == 0)
-        k_bitsums<double2><<<sh.grid, NT, 0, s>>>((const double2*)st, n, sh.g, sh.nr, (double2*)partials);
-    else
-        k_bitsums<double><<<sh.grid, NT, 0, s>>>((const double2*)st, n, sh.g, sh.nr, (double*)partials);
-    return cudaGetLastError();
-}
+namespace {
 
-cudaError_t launch_bitsums_c128_shape(const void* st, int n, int g, int nr, void* partials, cudaStream_t s) {
+template <typename V, typename S, bool SCALE>
+cudaError_t bitsums(S* st, int n, int g, int nr, void* partials, void* out, const double* scale,
+                    const int* err, int* err_out, cudaStream_t s, int first = 0) {
     if (nr < 0 || nr > MAXR || g < 0) return cudaErrorInvalidValue;
-    k_bitsums<double2><<<1 << g, NT, 0, s>>>((const double2*)st, n, g, nr, (double2*)partials);
+    if (n >= 12 ? n != 12 + g + nr : g + nr != 0) return cudaErrorInvalidValue;
+    const size_t smem = nr ? (sizeof(V) * (NT / 32)) << nr : 0;
+    V* dst = (V*)(g + nr ? partials : out);
+    k_bitsums<V, S, SCALE><<<1u << g, NT, smem, s>>>(st, n, g, nr, dst, scale, err, err_out);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || g + nr == 0) return e;
+    k_bitsums_finish<V><<<1 + 2 * n - first, NT, 0, s>>>((const V*)partials, g, first, (V*)out);
     return cudaGetLastError();
 }
 
-cudaError_t launch_probs_c128(const void* st, uint64_t dim, double* out, cudaStream_t s) {
-    uint64_t blocks = (dim + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    k_probs<double2><<<(unsigned)blocks, 256, 0, s>>>((const double2*)st, dim, out);
-    return cudaGetLastError();
+}  // namespace
+
+cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* partials, void* out, const int* err,
+                           int* err_out, cudaStream_t s) {
+    const BitSumShape sh = bitsum_shape(n);
+    if (prec == 0) {
+        double2* p = (double2*)const_cast<void*>(st);
+        return kind == 0 ? bitsums<double2, double2, false>(p, n, sh.g, sh.nr, partials, out, nullptr, err, err_out, s)
+                         : bitsums<double, double2, false>(p, n, sh.g, sh.nr, partials, out, nullptr, err, err_out, s);
+    }
+    float2* p = (float2*)const_cast<void*>(st);
+    return kind == 0 ? bitsums<double2, float2, false>(p, n, sh.g, sh.nr, partials, out, nullptr, err, err_out, s)
+                     : bitsums<double, float2, false>(p, n, sh.g, sh.nr, partials, out, nullptr, err, err_out, s);
 }
 
-cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* partials, cudaStream_t s) {
-    if (prec == 0) return launch_bitsums_c128(st, n, kind, partials, s);
-    BitSumShape sh = bitsum_shape(n);
-    if (sh.nr > MAXR) return cudaErrorInvalidValue;
-    if (kind == 0)
-        k_bitsums<double2, float2><<<sh.grid, NT, 0, s>>>((const float2*)st, n, sh.g, sh.nr, (double2*)partials);
-    else
-        k_bitsums<double, float2><<<sh.grid, NT, 0, s>>>((const float2*)st, n, sh.g, sh.nr, (double*)partials);
-    return cudaGetLastError();
+cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, void* partials, void* out, const int* err,
+                                      int* err_out, cudaStream_t s) {
+    const cudaError_t e = launch_norm_c64(st, n, scratch, s);
+    if (e != cudaSuccess) return e;
+    const BitSumShape sh = bitsum_shape(n);
+    return bitsums<double2, float2, true>((float2*)st, n, sh.g, sh.nr, partials, out,
+                                          (const double*)scratch + RN_GRID, err, err_out, s);
+}
+
+cudaError_t launch_bitsums_c128_shape(const void* st, int n, int g, int nr, void* partials, void* out,
+                                      cudaStream_t s) {
+    return bitsums<double2, double2, false>((double2*)const_cast<void*>(st), n, g, nr, partials, out, nullptr, nullptr, nullptr,
+                                           s, 1);
 }
 
 cudaError_t launch_probs(const void* st, int prec, uint64_t dim, double* out, cudaStream_t s) {
-    if (prec == 0) return launch_probs_c128(st, dim, out, s);
     uint64_t blocks = (dim + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    k_probs<float2><<<(unsigned)blocks, 256, 0, s>>>((const float2*)st, dim, out);
+    if (prec == 0) k_probs<double2><<<(unsigned)blocks, 256, 0, s>>>((const double2*)st, dim, out);
+    else k_probs<float2><<<(unsigned)blocks, 256, 0, s>>>((const float2*)st, dim, out);
     return cudaGetLastError();
 }
 

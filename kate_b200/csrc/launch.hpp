@@ -22,7 +22,6 @@ cudaError_t launch_set_basis0(void* st, uint64_t dim, int prec, cudaStream_t s);
 cudaError_t launch_init_product(void* st, int n, const ProductInit& P, int prec, cudaStream_t s);
 cudaError_t launch_pass_generic(void* st, int prec, const DevPass& p, const DevOp* ops, const void* pool, int grid,
                                 cudaStream_t s);
-cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* partials, cudaStream_t s);
 cudaError_t launch_probs(const void* st, int prec, uint64_t dim, double* out, cudaStream_t s);
 // Renormalisation of a complex64 state (n >= 1 qubits): ||psi||^2 reduced in
 // FP64 on the device, then every amplitude multiplied by 1 / ||psi||. The
@@ -30,13 +29,15 @@ cudaError_t launch_probs(const void* st, int prec, uint64_t dim, double* out, cu
 // then ||psi||^2 and 1 / ||psi|| as doubles 0 and 1 after the partials
 // (offset renorm_result_offset()), then a counter.
 size_t renorm_scratch_bytes();
-// Inverse-CDF sampling on the device (k_sample.cu): unif holds `shots`
-// uniforms in [0, 1), ascending; out[s] receives the physical index of the
-// first amplitude whose FP64 cumulative probability exceeds unif[s] * total.
-// scratch: sample_scratch_doubles(n) doubles.
+// Inverse-CDF sampling on the device (k_sample.cu): out[k] receives shot k of
+// `seed` as a basis index in program labels, label q read from physical bit
+// phys[q]. scratch: sample_scratch_doubles(n) doubles.
+struct SampleLabels {
+    uint8_t phys[KATE_MAX_QUBITS];
+};
 size_t sample_scratch_doubles(int n);
-cudaError_t launch_sample(const void* st, int prec, int n, const double* unif, int shots, double* scratch,
-                          uint64_t* out, cudaStream_t s);
+cudaError_t launch_sample(const void* st, int prec, int n, uint64_t seed, int shots, const SampleLabels& L,
+                          double* scratch, uint64_t* out, cudaStream_t s);
 // Device gate merger (k_merge.cu): out[b] is the product of blocks[b] as one
 // dense gate on the sorted union of its qubits (at most 10), bit-identical
 // to merge_gates (circuit.hpp); all blocks in one launch on `device`, then
@@ -44,6 +45,7 @@ cudaError_t launch_sample(const void* st, int prec, int n, const double* unif, i
 struct Gate;
 std::string merge_gates_device(const std::vector<std::vector<Gate>>& blocks, int device, cudaStream_t stream,
                                std::vector<Gate>* out);
+cudaError_t launch_norm_c64(const void* st, int n, void* scratch, cudaStream_t s);  // ||psi||^2 only
 constexpr size_t renorm_result_offset() { return 148 * 4 * sizeof(double); }
 cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s);
 
@@ -86,21 +88,30 @@ cudaError_t launch_batch(void* arena, int prec, const BatchTask* tasks, int ntas
                          unsigned long long wait_ns = 5000000000ull, int tensor_blocks = 0);
 int batch_grid(int device, int prec, bool tensor_blocks = false);
 
-// Bit sums: per CTA, for every local bit, the sum over amplitudes with the
-// bit 0 and with the bit 1, plus the total. kind 0 sums amplitudes (double2
-// partials), kind 1 sums |a|^2 (double partials). Returns the grid shape.
+// Bit sums (k_measure.cu): out[0] = total, out[1 + 2b + v] = the sum over the
+// amplitudes whose physical index bit b is v; kind 0 sums amplitudes (double2
+// values), kind 1 |a|^2 (double values). `out` holds max(25, 1 + 2n) values,
+// `partials` grid * nout of the shape below (CTA partials). *err_out receives
+// *err (the error flag of the kernels before; both nullable): out and err_out
+// may lie in pinned host memory, so that a caller waits once and copies
+// nothing.
 struct BitSumShape {
     int grid;   // CTAs (2^g)
     int g;      // coset bits handled by the grid
-    int nr;     // round bits handled per thread
+    int nr;     // round bits handled per CTA
     int nout;   // partial values per CTA
 };
 BitSumShape bitsum_shape(int n);
-cudaError_t launch_bitsums_c128(const void* st, int n, int kind, void* partials, cudaStream_t s);
-// Amplitude bit sums with an explicit shape: 2^g CTAs, nr round bits per
-// thread (n = 12 + g + nr when n >= 12), partials of 1 + 2 * (12 + nr)
-// double2 per CTA.
-cudaError_t launch_bitsums_c128_shape(const void* st, int n, int g, int nr, void* partials, cudaStream_t s);
-cudaError_t launch_probs_c128(const void* st, uint64_t dim, double* out, cudaStream_t s);
+cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* partials, void* out, const int* err,
+                           int* err_out, cudaStream_t s);
+// launch_renorm_c64 and the amplitude bit sums (kind 0) of the rescaled
+// state, which the rescaling pass adds up as it goes.
+cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, void* partials, void* out, const int* err,
+                                      int* err_out, cudaStream_t s);
+// Amplitude bit sums of a complex128 state with an explicit shape: 2^g CTAs,
+// 2^nr rounds each (n = 12 + g + nr when n >= 12, nr <= 8). When g + nr > 0
+// the total out[0] is not written.
+cudaError_t launch_bitsums_c128_shape(const void* st, int n, int g, int nr, void* partials, void* out,
+                                      cudaStream_t s);
 
 }  // namespace kate

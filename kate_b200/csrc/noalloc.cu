@@ -47,7 +47,7 @@ namespace kate {
 namespace {
 
 constexpr int kGridBits = 10;                   // 1024 CTAs
-constexpr int kMaxRoundBits = 8;                // rounds per thread (k_bitsums)
+constexpr int kMaxRoundBits = 8;                // rounds per CTA (k_bitsums)
 constexpr int kPartsPerCta = 1 + 2 * (12 + kMaxRoundBits);
 constexpr int kPartials = (1 << kGridBits) * kPartsPerCta;
 constexpr int kFinal = 2 * KATE_NOALLOC_MAX_QUBITS;
@@ -56,26 +56,6 @@ constexpr int kFinal = 2 * KATE_NOALLOC_MAX_QUBITS;
 // bit = 1) pair of every physical bit.
 static __device__ __align__(256) double2 g_scratch[kPartials + kFinal];
 static_assert(sizeof(g_scratch) <= KATE_NOALLOC_SCRATCH_BYTES, "scratch size");
-
-// Adds the per-CTA partials of k_bitsums into one (bit 0, bit 1) sum pair
-// per physical bit, in CTA order. One thread per output.
-__global__ void k_finish(const double2* __restrict__ part, int n, int g, int nout, double2* __restrict__ out) {
-    const int o = threadIdx.x;
-    if (o >= 2 * n) return;
-    const int b = o / 2, one = o & 1;
-    double2 s = make_double2(0.0, 0.0);
-    const int grid = 1 << g;
-    for (int c = 0; c < grid; c++) {
-        const double2* pc = part + (size_t)c * nout;
-        double2 v;
-        if (b < 12) v = pc[1 + 2 * b + one];
-        else if (b < 12 + g) v = ((((c >> (b - 12)) & 1) == one) ? pc[0] : make_double2(0.0, 0.0));
-        else v = pc[1 + 2 * (12 + (b - 12 - g)) + one];
-        s.x += v.x;
-        s.y += v.y;
-    }
-    out[o] = s;
-}
 
 kate_status fail(kate_status st, const std::string& m) {
     set_last_error(m);
@@ -158,15 +138,13 @@ extern "C" kate_status kate_proba_state_noalloc(const void* d_state, size_t stat
     double2* fin = part + kPartials;
     const int g = n <= 12 ? 0 : (n - 12 < kGridBits ? n - 12 : kGridBits);
     const int nr = n <= 12 ? 0 : n - 12 - g;
-    const int nout = 1 + 2 * (12 + nr);
+    // Output v of bit b at out[1 + 2b + v]; one CTA (n <= 12) writes its total
+    // at out[0] too.
+    double2* out = g + nr ? fin - 1 : fin;
     cudaStream_t s = (cudaStream_t)stream;
-    ce = launch_bitsums_c128_shape(d_state, n, g, nr, part, s);
-    if (ce == cudaSuccess) {
-        k_finish<<<1, 64, 0, s>>>(part, n, g, nout, fin);
-        ce = cudaGetLastError();
-    }
+    ce = launch_bitsums_c128_shape(d_state, n, g, nr, part, out, s);
     double2 sums[kFinal];
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(sums, fin, sizeof(double2) * 2 * n, cudaMemcpyDeviceToHost, s);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(sums, out + 1, sizeof(double2) * 2 * n, cudaMemcpyDeviceToHost, s);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
     if (ce != cudaSuccess) return fail(KATE_ECUDA, std::string("measurement: ") + cudaGetErrorString(ce));
     // The reference's formula (HIPcode/simulator.hpp:519-535), its Complex

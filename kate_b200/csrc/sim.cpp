@@ -45,9 +45,16 @@ struct SimImpl {
     void* d_part = nullptr;
     void* d_bimg = nullptr;   // complex64 block operand images
     int* d_err = nullptr;     // set by kernels whose bounded waits gave up
+    // Measurement results: the error flag, then (at +16 bytes) the bit sums,
+    // or samples. Pinned host memory that kernels write directly, or, when
+    // none is left, device memory copied to `host_out` after the kernel.
+    char* pinned = nullptr;
+    char* d_res = nullptr;
+    std::vector<char> host_out;
+    char* d_samp = nullptr;   // sampling workspace, kept once used
+    size_t samp_bytes = 0;
     void* d_norm = nullptr;   // complex64: renormalisation scratch and result
     bool renormed = false;    // a complex64 run has been renormalised
-    size_t part_bytes = 0;
     std::vector<DevPass> hpasses;
     cudaStream_t stream = nullptr;
     std::vector<int> phys;  // current layout: logical -> physical
@@ -102,37 +109,78 @@ struct SimImpl {
         return "";
     }
 
-    // Sums over amplitudes (kind 0) or probabilities (kind 1) for every
-    // physical bit; s0/s1 are 2 doubles per bit for kind 0, 1 for kind 1.
-    std::string bit_sums(int kind, std::vector<double>& s0, std::vector<double>& s1, double* total) {
-        BitSumShape sh = bitsum_shape(n);
-        const int w = kind == 0 ? 2 : 1;
-        std::vector<double> h((size_t)sh.grid * sh.nout * w);
-        KCHECK(launch_bitsums(d_state, precision, n, kind, d_part, stream));
-        KCHECK(cudaMemcpyAsync(h.data(), d_part, h.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
-        KCHECK(cudaStreamSynchronize(stream));
-        s0.assign((size_t)n * w, 0.0);
-        s1.assign((size_t)n * w, 0.0);
-        std::vector<double> tot(w, 0.0);
-        for (int c = 0; c < sh.grid; c++) {
-            const double* pc = h.data() + (size_t)c * sh.nout * w;
-            for (int k = 0; k < w; k++) tot[k] += pc[k];
-            for (int b = 0; b < n; b++) {
-                int slot;
-                if (b < 12) slot = b;
-                else if (b < 12 + sh.g) {
-                    bool one = (c >> (b - 12)) & 1;
-                    for (int k = 0; k < w; k++) (one ? s1 : s0)[(size_t)b * w + k] += pc[k];
-                    continue;
-                } else slot = 12 + (b - 12 - sh.g);
-                for (int k = 0; k < w; k++) {
-                    s0[(size_t)b * w + k] += pc[(size_t)(1 + 2 * slot) * w + k];
-                    s1[(size_t)b * w + k] += pc[(size_t)(2 + 2 * slot) * w + k];
-                }
-            }
+    // Where a measurement's kernels write (flag first) and its bytes.
+    size_t res_bytes() const { return 16 + std::max<size_t>(25, 1 + 2 * (size_t)n) * sizeof(double2); }
+    char* res() const { return pinned ? pinned : d_res; }
+    void* res_sums() const { return res() + 16; }
+    int* res_flag() const { return (int*)res(); }
+
+    // Waits for the bit sums queued on the simulator's stream and the work
+    // before them; *out points at the sums on the host. `check`: the flag was
+    // written with them and is looked at.
+    std::string fetch(const char** out, bool check) {
+        if (!pinned) {
+            host_out.resize(res_bytes());
+            KCHECK(cudaMemcpyAsync(host_out.data(), d_res, host_out.size(), cudaMemcpyDeviceToHost, stream));
         }
-        if (total) for (int k = 0; k < w; k++) total[k] = tot[k];
+        KCHECK(cudaStreamSynchronize(stream));
+        const char* r = pinned ? pinned : host_out.data();
+        int flag = 0;
+        if (check) std::memcpy(&flag, r, sizeof flag);
+        if (flag) return timed_out();
+        *out = r + 16;
         return "";
+    }
+    std::string timed_out() {
+        cudaMemset(d_err, 0, sizeof(int));
+        return "timed out: a bounded device wait gave up (tensor-core completion not observed)";
+    }
+
+    // Sums over amplitudes (kind 0, two doubles per value) or probabilities
+    // (kind 1, one): *sums holds the total, then the sums with physical bit b
+    // 0 and 1 at values 1 + 2b and 2 + 2b.
+    std::string bit_sums(int kind, const double** sums) {
+        KCHECK(launch_bitsums(d_state, precision, n, kind, d_part, res_sums(), nullptr, nullptr, stream));
+        const char* r = nullptr;
+        std::string e = fetch(&r, false);
+        *sums = (const double*)r;
+        return e;
+    }
+
+    // The reference's measurement from the amplitude sums
+    // (HIPcode/simulator.hpp:519-535 with its Complex division, norm and
+    // angle, backendagnosticcode/basic_host_types.hpp:28-57).
+    void proba_from_sums(const double* sums, double* out) const {
+        const double p = std::pow(kSqrt2, (double)n);
+        auto cdiv = [](double ar, double ai, double br, double bi, double& rr, double& ri) {
+            double d = br * br + bi * bi;
+            rr = (ar * br + ai * bi) / d;
+            ri = (br * ai - ar * bi) / d;
+        };
+        for (int x = 0; x < n; x++) {
+            const int b = phys_of_label(x);
+            const double *s0 = sums + 2 * (1 + 2 * b), *s1 = s0 + 2;
+            double v0r, v0i, v1r, v1i;
+            cdiv(s0[0], s0[1], p, 0.0, v0r, v0i);
+            cdiv(s1[0], s1[1], p, 0.0, v1r, v1i);
+            double n0 = std::sqrt(v0r * v0r + v0i * v0i), n1 = std::sqrt(v1r * v1r + v1i * v1i);
+            double teta, phi;
+            if (n0 < 0.0000000000001) {
+                teta = 1;
+                phi = 0;
+            } else if (n1 < 0.00000000000001) {
+                teta = 0;
+                phi = 0;
+            } else {
+                teta = std::atan(n1 / n0) / (kPi / 2);
+                double qr, qi;
+                cdiv(v1r, v1i, v0r, v0i, qr, qi);
+                phi = std::atan(qi / qr);
+            }
+            const int o = plan.final_inverse_permutation.empty() ? x : plan.final_inverse_permutation[x];
+            out[2 * o] = teta;
+            out[2 * o + 1] = phi;
+        }
     }
 };
 
@@ -223,9 +271,13 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
     if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(error flag)", ce));
     cudaMemset(impl->d_err, 0, sizeof(int));
     BitSumShape sh = bitsum_shape(impl->n);
-    impl->part_bytes = (size_t)sh.grid * sh.nout * 2 * sizeof(double);
-    ce = cudaMalloc(&impl->d_part, impl->part_bytes);
+    ce = cudaMalloc(&impl->d_part, (size_t)sh.grid * sh.nout * 2 * sizeof(double));
     if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(partials)", ce));
+    impl->pinned = (char*)pinned_take();
+    if (!impl->pinned) {
+        ce = cudaMalloc(&impl->d_res, impl->res_bytes());
+        if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(results)", ce));
+    }
     ce = cached_malloc(&impl->d_state, impl->dim() * impl->amp_bytes(), device);
     if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(state)", ce));
     impl->grid = generic_pass_grid(impl->n, std::min(impl->opt.max_tile, impl->n), device);
@@ -354,6 +406,9 @@ Simulator::~Simulator() {
     cudaFree(d_->d_sops);
     cudaFree(d_->d_pool);
     cudaFree(d_->d_part);
+    pinned_give(d_->pinned);
+    cudaFree(d_->d_res);
+    cudaFree(d_->d_samp);
     cudaFree(d_->d_bimg);
     cudaFree(d_->d_err);
     cudaFree(d_->d_norm);
@@ -425,7 +480,20 @@ std::string Simulator::enqueue_init(void* stream, const double* tp) {
     return "";
 }
 
-std::string Simulator::enqueue_passes(void* stream) {
+std::string Simulator::execute(const double* tp_in, double* tp_out) {
+    SimImpl& S = *d_;
+    KCHECK(cudaSetDevice(S.device));
+    std::string e = enqueue_init(S.stream, tp_in);
+    if (e.empty()) e = enqueue_passes(S.stream, tp_out != nullptr);
+    if (!e.empty()) return e;
+    if (!tp_out) return synchronize();
+    const char* r = nullptr;
+    e = S.fetch(&r, true);
+    if (e.empty()) S.proba_from_sums((const double*)r, tp_out);
+    return e;
+}
+
+std::string Simulator::enqueue_passes(void* stream, bool sums) {
     SimImpl& S = *d_;
     cudaStream_t st = (cudaStream_t)stream;
     const bool zs = S.zero_start, ps = S.prod_start;
@@ -440,8 +508,13 @@ std::string Simulator::enqueue_passes(void* stream) {
     }
     if (S.precision == 1) {
         // Complex64: ||psi|| in FP64, then the state rescaled to norm 1.
-        KCHECK(launch_renorm_c64(S.d_state, S.n, S.d_norm, st));
+        if (sums)
+            KCHECK(launch_renorm_bitsums_c64(S.d_state, S.n, S.d_norm, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
+        else
+            KCHECK(launch_renorm_c64(S.d_state, S.n, S.d_norm, st));
         S.renormed = true;
+    } else if (sums) {
+        KCHECK(launch_bitsums(S.d_state, 0, S.n, 0, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
     }
     S.phys = S.plan.final_phys;
     S.has_state = true;
@@ -495,65 +568,29 @@ std::string Simulator::synchronize() {
     KCHECK(cudaStreamSynchronize(d_->stream));
     int flag = 0;
     KCHECK(cudaMemcpy(&flag, d_->d_err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (flag) {
-        cudaMemset(d_->d_err, 0, sizeof(int));
-        return "timed out: a bounded device wait gave up (tensor-core completion not observed)";
-    }
-    return "";
+    return flag ? d_->timed_out() : "";
 }
 
 std::string Simulator::proba_state(double* out) {
     SimImpl& S = *d_;
     if (!S.has_state) return "no state: execute the simulator first";
     KCHECK(cudaSetDevice(S.device));
-    std::vector<double> s0, s1;
-    std::string e = S.bit_sums(0, s0, s1, nullptr);
-    if (!e.empty()) return e;
-    // HIPcode/simulator.hpp:519-535 with the reference's Complex division,
-    // norm and angle (backendagnosticcode/basic_host_types.hpp:28-57).
-    const int n = S.n;
-    const double p = std::pow(kSqrt2, (double)n);
-    auto cdiv = [](double ar, double ai, double br, double bi, double& rr, double& ri) {
-        double d = br * br + bi * bi;
-        rr = (ar * br + ai * bi) / d;
-        ri = (br * ai - ar * bi) / d;
-    };
-    for (int x = 0; x < n; x++) {
-        int b = S.phys_of_label(x);
-        double v0r, v0i, v1r, v1i;
-        cdiv(s0[2 * b], s0[2 * b + 1], p, 0.0, v0r, v0i);
-        cdiv(s1[2 * b], s1[2 * b + 1], p, 0.0, v1r, v1i);
-        double n0 = std::sqrt(v0r * v0r + v0i * v0i), n1 = std::sqrt(v1r * v1r + v1i * v1i);
-        double teta, phi;
-        if (n0 < 0.0000000000001) {
-            teta = 1;
-            phi = 0;
-        } else if (n1 < 0.00000000000001) {
-            teta = 0;
-            phi = 0;
-        } else {
-            teta = std::atan(n1 / n0) / (kPi / 2);
-            double qr, qi;
-            cdiv(v1r, v1i, v0r, v0i, qr, qi);
-            phi = std::atan(qi / qr);
-        }
-        int o = S.plan.final_inverse_permutation.empty() ? x : S.plan.final_inverse_permutation[x];
-        out[2 * o] = teta;
-        out[2 * o + 1] = phi;
-    }
-    return "";
+    const double* sums = nullptr;
+    std::string e = S.bit_sums(0, &sums);
+    if (e.empty()) S.proba_from_sums(sums, out);
+    return e;
 }
 
 std::string Simulator::expect_z(double* out) {
     SimImpl& S = *d_;
     if (!S.has_state) return "no state: execute the simulator first";
     KCHECK(cudaSetDevice(S.device));
-    std::vector<double> s0, s1;
-    std::string e = S.bit_sums(1, s0, s1, nullptr);
+    const double* sums = nullptr;
+    std::string e = S.bit_sums(1, &sums);
     if (!e.empty()) return e;
     for (int x = 0; x < S.n; x++) {
-        int b = S.phys_of_label(x);
-        out[x] = s0[b] - s1[b];
+        const double* s0 = sums + 1 + 2 * S.phys_of_label(x);
+        out[x] = s0[0] - s0[1];
     }
     return "";
 }
@@ -618,45 +655,27 @@ std::string Simulator::sample(int shots, uint64_t seed, uint64_t* out) {
     if (!S.has_state) return "no state: execute the simulator first";
     if (shots == 0) return "";
     KCHECK(cudaSetDevice(S.device));
-    // Uniforms u = (splitmix64 >> 11) * 2^-53 in draw order (the generator
-    // the server's samples use), sorted for the device with their shot index.
-    std::vector<std::pair<double, int>> us((size_t)shots);
-    uint64_t sm = seed;
-    for (int k = 0; k < shots; k++) {
-        sm += 0x9E3779B97F4A7C15ull;
-        uint64_t z = sm;
-        z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-        z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-        z ^= z >> 31;
-        us[(size_t)k] = {(double)(z >> 11) * (1.0 / 9007199254740992.0), k};
+    // Samples go straight to pinned memory when they fit, else to the end of
+    // the workspace and from there in one copy.
+    const size_t out_bytes = (size_t)shots * sizeof(uint64_t);
+    const bool direct = S.pinned && out_bytes <= kPinnedSlotBytes;
+    const size_t scr = sample_scratch_doubles(S.n) * sizeof(double);
+    const size_t need = scr + (direct ? 0 : out_bytes);
+    if (S.samp_bytes < need) {
+        KCHECK(cudaStreamSynchronize(S.stream));
+        cudaFree(S.d_samp);
+        S.d_samp = nullptr;
+        S.samp_bytes = 0;
+        KCHECK(cudaMalloc(&S.d_samp, need));
+        S.samp_bytes = need;
     }
-    std::sort(us.begin(), us.end());
-    std::vector<double> u((size_t)shots);
-    for (int k = 0; k < shots; k++) u[(size_t)k] = us[(size_t)k].first;
-    const size_t nscr = sample_scratch_doubles(S.n);
-    char* buf = nullptr;
-    const size_t bytes = (nscr + (size_t)shots) * sizeof(double) + (size_t)shots * sizeof(uint64_t);
-    KCHECK(cudaMallocAsync((void**)&buf, bytes, S.stream));
-    double* d_scr = (double*)buf;
-    double* d_u = d_scr + nscr;
-    uint64_t* d_out = (uint64_t*)(d_u + shots);
-    std::vector<uint64_t> phys((size_t)shots);
-    cudaError_t ce = cudaMemcpyAsync(d_u, u.data(), (size_t)shots * sizeof(double), cudaMemcpyHostToDevice, S.stream);
-    if (ce == cudaSuccess) ce = launch_sample(S.d_state, S.precision, S.n, d_u, shots, d_scr, d_out, S.stream);
-    if (ce == cudaSuccess)
-        ce = cudaMemcpyAsync(phys.data(), d_out, (size_t)shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, S.stream);
-    cudaFreeAsync(buf, S.stream);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(S.stream);
-    if (ce != cudaSuccess) return cuda_err("sample", ce);
-    // Physical index -> index in the reference's qubit labels.
-    std::vector<int> pb(S.n);
-    for (int x = 0; x < S.n; x++) pb[x] = S.phys_of_label(x);
-    for (int k = 0; k < shots; k++) {
-        const uint64_t v = phys[(size_t)k];
-        uint64_t lab = 0;
-        for (int x = 0; x < S.n; x++) lab |= ((v >> pb[x]) & 1ull) << x;
-        out[us[(size_t)k].second] = lab;
-    }
+    SampleLabels L{};
+    for (int x = 0; x < S.n; x++) L.phys[x] = (uint8_t)S.phys_of_label(x);
+    uint64_t* dst = (uint64_t*)(direct ? S.pinned : S.d_samp + scr);
+    KCHECK(launch_sample(S.d_state, S.precision, S.n, seed, shots, L, (double*)S.d_samp, dst, S.stream));
+    if (!direct) KCHECK(cudaMemcpyAsync(out, dst, out_bytes, cudaMemcpyDeviceToHost, S.stream));
+    KCHECK(cudaStreamSynchronize(S.stream));
+    if (direct) std::memcpy(out, S.pinned, out_bytes);
     return "";
 }
 

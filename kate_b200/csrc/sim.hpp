@@ -22,6 +22,9 @@ public:
 
     std::string run_async(void* stream, const double* theta_phi_in);  // init + all passes, no sync
     std::string synchronize();
+    // run_async on the simulator's stream, then the measurement queued behind
+    // it and one wait for both. tp_in / tp_out nullable.
+    std::string execute(const double* tp_in, double* tp_out);
     // init + passes with CUDA events between them, then the measurement on
     // the host clock: ms[0] init, ms[1] group passes, ms[2] proba_state,
     // ms[3] number of passes. tp_in / tp_out nullable.
@@ -55,7 +58,8 @@ public:
 private:
     // Queue the initial state / every group pass on stream st (cudaStream_t).
     std::string enqueue_init(void* st, const double* tp);
-    std::string enqueue_passes(void* st);
+    // With `sums` the amplitude sums of the final state are queued too.
+    std::string enqueue_passes(void* st, bool sums = false);
     SimImpl* d_ = nullptr;
 };
 
