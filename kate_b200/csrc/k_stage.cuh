@@ -84,10 +84,39 @@ __device__ __forceinline__ C2 row2(C2 u0, C2 u1, C2 x, C2 y) {
     return r;
 }
 
-template <int B, typename C2>
-__device__ __forceinline__ void reg_u(C2 (&a)[16], C2 u00, C2 u01, C2 u10, C2 u11) {
+// Register ops on N amplitudes per thread (16; 4 or 8 in the one-CTA kernel
+// of small states), register-index bit B.
+
+// f(bit) with the register bit b < log2(N) as a compile-time constant.
+template <int V>
+struct BitC {
+    static constexpr int value = V;
+};
+template <int N, typename F>
+__device__ __forceinline__ void on_bit(int b, F&& f) {
+    if constexpr (N == 4) {
+        if (b == 0) f(BitC<0>{});
+        else f(BitC<1>{});
+    } else if constexpr (N == 8) {
+        switch (b) {
+        case 0: f(BitC<0>{}); break;
+        case 1: f(BitC<1>{}); break;
+        default: f(BitC<2>{}); break;
+        }
+    } else {
+        switch (b) {
+        case 0: f(BitC<0>{}); break;
+        case 1: f(BitC<1>{}); break;
+        case 2: f(BitC<2>{}); break;
+        default: f(BitC<3>{}); break;
+        }
+    }
+}
+
+template <int B, int N, typename C2>
+__device__ __forceinline__ void reg_u(C2 (&a)[N], C2 u00, C2 u01, C2 u10, C2 u11) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         const int k = j | (1 << B);
         const C2 x = a[j], y = a[k];
@@ -98,10 +127,10 @@ __device__ __forceinline__ void reg_u(C2 (&a)[16], C2 u00, C2 u01, C2 u10, C2 u1
 
 // Dense two-qubit gate on register bits A (matrix index bit 0) and B (bit
 // 1), matrix M (4x4 row-major, complex128 only).
-template <int A, int B>
-__device__ __forceinline__ void reg_u2(double2 (&a)[16], const double2* M) {
+template <int A, int B, int N>
+__device__ __forceinline__ void reg_u2(double2 (&a)[N], const double2* M) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if (((j >> A) & 1) || ((j >> B) & 1)) continue;
         const int r1 = j | (1 << A), r2 = j | (1 << B), r3 = j | (1 << A) | (1 << B);
         const double2 x0 = a[j], x1 = a[r1], x2 = a[r2], x3 = a[r3];
@@ -120,11 +149,11 @@ __device__ __forceinline__ void reg_u2(double2 (&a)[16], const double2* M) {
     }
 }
 
-template <int B, typename C2>
-__device__ __forceinline__ void reg_h(C2 (&a)[16]) {
+template <int B, int N, typename C2>
+__device__ __forceinline__ void reg_h(C2 (&a)[N]) {
     using R = typename Amp<C2>::R;
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         const int k = j | (1 << B);
         const C2 x = a[j], y = a[k];
@@ -140,10 +169,10 @@ __device__ __forceinline__ void reg_h(C2 (&a)[16]) {
     }
 }
 
-template <int B, typename C2>
-__device__ __forceinline__ void reg_x(C2 (&a)[16], uint32_t creg) {
+template <int B, int N, typename C2>
+__device__ __forceinline__ void reg_x(C2 (&a)[N], uint32_t creg) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         if (((uint32_t)j & creg) != creg) continue;
         const int k = j | (1 << B);
@@ -154,11 +183,11 @@ __device__ __forceinline__ void reg_x(C2 (&a)[16], uint32_t creg) {
 }
 
 // Real 2x2 [[a, b], [c, d]]: 4 FMA-class ops per amplitude.
-template <int B, typename C2, typename R>
-__device__ __forceinline__ void reg_ur(C2 (&a)[16], R u00, R u01, R u10, R u11) {
+template <int B, int N, typename C2, typename R>
+__device__ __forceinline__ void reg_ur(C2 (&a)[N], R u00, R u01, R u10, R u11) {
     using A = Amp<C2>;
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         const int k = j | (1 << B);
         const C2 x = a[j], y = a[k];
@@ -173,11 +202,11 @@ __device__ __forceinline__ void reg_ur(C2 (&a)[16], R u00, R u01, R u10, R u11) 
 }
 
 // [[a, ib], [ic, d]] with a, b, c, d real (RX-like): 4 FMA-class ops per amplitude.
-template <int B, typename C2, typename R>
-__device__ __forceinline__ void reg_ux(C2 (&a)[16], R u00, R u01i, R u10i, R u11) {
+template <int B, int N, typename C2, typename R>
+__device__ __forceinline__ void reg_ux(C2 (&a)[N], R u00, R u01i, R u10i, R u11) {
     using A = Amp<C2>;
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         const int k = j | (1 << B);
         const C2 x = a[j], y = a[k];
@@ -198,11 +227,11 @@ __device__ __forceinline__ void reg_ux(C2 (&a)[16], R u00, R u01i, R u10i, R u11
 //   F = 1 (URB): t0 x0 + x1,    t1 x1 - x0
 //   F = 2 (UXA): x0 + i t0 x1,  x1 + i t1 x0
 //   F = 3 (UXB): x1 - i t0 x0,  x0 - i t1 x1
-template <int F, int B, typename C2, typename R>
-__device__ __forceinline__ void reg_rot(C2 (&a)[16], R t0, R t1) {
+template <int F, int B, int N, typename C2, typename R>
+__device__ __forceinline__ void reg_rot(C2 (&a)[N], R t0, R t1) {
     using A = Amp<C2>;
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         const int k = j | (1 << B);
         const C2 x = a[j], y = a[k];
@@ -239,21 +268,16 @@ __device__ __forceinline__ void reg_rot(C2 (&a)[16], R t0, R t1) {
     }
 }
 
-template <int F, typename C2, typename R>
-__device__ __forceinline__ void reg_rot_bit(C2 (&a)[16], int b, R t0, R t1) {
-    switch (b) {
-    case 0: reg_rot<F, 0>(a, t0, t1); break;
-    case 1: reg_rot<F, 1>(a, t0, t1); break;
-    case 2: reg_rot<F, 2>(a, t0, t1); break;
-    default: reg_rot<F, 3>(a, t0, t1); break;
-    }
+template <int F, int N, typename C2, typename R>
+__device__ __forceinline__ void reg_rot_bit(C2 (&a)[N], int b, R t0, R t1) {
+    on_bit<N>(b, [&](auto B) { reg_rot<F, B.value>(a, t0, t1); });
 }
 
 // Controlled NOT with a per-thread condition: selects, no branches.
-template <int B, typename C2>
-__device__ __forceinline__ void reg_xs(C2 (&a)[16], uint32_t creg, bool go) {
+template <int B, int N, typename C2>
+__device__ __forceinline__ void reg_xs(C2 (&a)[N], uint32_t creg, bool go) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) {
+    for (int j = 0; j < N; j++) {
         if ((j >> B) & 1) continue;
         if (((uint32_t)j & creg) != creg) continue;
         const int k = j | (1 << B);
@@ -551,15 +575,20 @@ __device__ __forceinline__ uint32_t plain_off(uint32_t s) { return ops::swz(s >>
 // 256-byte runs), so the first stage loads through plain_off, and its
 // stores, which use the swizzled order, wait behind a barrier for every
 // thread's first-stage loads. D->okL is not used in this mode.
-template <typename C2, bool SM, int MAXK = 5, int MODE = 0>
-__device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, uint32_t tb, C2* tile, uint64_t cbase,
+// N: amplitudes per thread. TT: the tables' type (ops, mats and stab are
+// read). A tile of fewer qubits (k_small.cu) gives its tile bits, its CTA's
+// threads and this thread's index among them for the shared-memory ops; t is
+// then the index within the program's 2^(tile bits) / N threads.
+template <typename C2, bool SM, int MAXK = 5, int MODE = 0, int N = 16, typename TT = TileTables<C2>>
+__device__ __forceinline__ void run_program(const TT& T, int nops, uint32_t tb, C2* tile, uint64_t cbase,
                                             const DevOp* __restrict__ sops, int sop0,
                                             const double2* __restrict__ pool, uint32_t t,
-                                            const DirectIO* D = nullptr, C2* __restrict__ gst = nullptr) {
+                                            const DirectIO* D = nullptr, C2* __restrict__ gst = nullptr,
+                                            int tile_bits = TB, int nthreads = NT, int tid = -1) {
     static_assert(MODE == 0 || (!SM && sizeof(C2) == 16), "the warp-specialised mode runs complex128 register programs");
     using A = Amp<C2>;
     using R = typename A::R;
-    C2 a[16];
+    C2 a[N];
     bool open = false;
     bool started = false;  // a stage has been loaded
     bool plain_open = false;  // MODE 1: the open stage was loaded from the plain-order tile
@@ -576,7 +605,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
         const uint16_t* tab = T.stab[si];
         const uint32_t v0 = tab[36], v1 = tab[37], v2 = tab[38], v3 = tab[39];
 #pragma unroll
-        for (int j = 0; j < 16; j++) A::sts(tb + reg_off(j, s0s, v0, v1, v2, v3), a[j]);
+        for (int j = 0; j < N; j++) A::sts(tb + reg_off(j, s0s, v0, v1, v2, v3), a[j]);
     };
     for (int k = 0; k < nops; k++) {
         const SOp op = T.ops[k];
@@ -592,7 +621,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
                     const uint32_t p0 = plain_off(tab[32]), p1 = plain_off(tab[33]), p2 = plain_off(tab[34]),
                                    p3 = plain_off(tab[35]), pl = plain_off(sl);
 #pragma unroll
-                    for (int j = 0; j < 16; j++) a[j] = A::lds(tb + reg_off(j, pl, p0, p1, p2, p3));
+                    for (int j = 0; j < N; j++) a[j] = A::lds(tb + reg_off(j, pl, p0, p1, p2, p3));
                     started = true;
                     plain_open = true;
                     s0s = s0;
@@ -608,7 +637,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
                     const uint32_t x = sl >> 4;
                     const uint64_t base = cbase ^ D->ml[x & 63u] ^ D->mh[x >> 6];
 #pragma unroll
-                    for (int j = 0; j < 16; j++) a[j] = __ldcg(gst + (base ^ D->lr[j]));
+                    for (int j = 0; j < N; j++) a[j] = __ldcg(gst + (base ^ D->lr[j]));
                     started = true;
                     s0s = s0;
                     lflip = 0;
@@ -622,7 +651,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
             else prog_bar<MODE>();
             const uint32_t w0 = tab[32], w1 = tab[33], w2 = tab[34], w3 = tab[35];
 #pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = A::lds(tb + reg_off(j, sl, w0, w1, w2, w3));
+            for (int j = 0; j < N; j++) a[j] = A::lds(tb + reg_off(j, sl, w0, w1, w2, w3));
             started = true;
             s0s = s0;
             lflip = 0;
@@ -645,43 +674,28 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
             }
             // The registers are dead until the next stage loads them.
 #pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = A::mk(0, 0);
+            for (int j = 0; j < N; j++) a[j] = A::mk(0, 0);
             __syncthreads();
             const DevOp d = sops[sop0 + op.idx];
-            ops::apply_op<C2, MAXK>(tile, TB, cbase, d, pool, (int)t, NT);
+            ops::apply_op<C2, MAXK>(tile, tile_bits, cbase, d, pool, tid < 0 ? (int)t : tid, nthreads);
             __syncthreads();
             break;
         }
         case SOP_U: {
             const C2 u00 = T.mats[op.idx], u01 = T.mats[op.idx + 1], u10 = T.mats[op.idx + 2], u11 = T.mats[op.idx + 3];
-            switch (op.a) {
-            case 0: reg_u<0>(a, u00, u01, u10, u11); break;
-            case 1: reg_u<1>(a, u00, u01, u10, u11); break;
-            case 2: reg_u<2>(a, u00, u01, u10, u11); break;
-            default: reg_u<3>(a, u00, u01, u10, u11); break;
-            }
+            on_bit<N>(op.a, [&](auto B) { reg_u<B.value>(a, u00, u01, u10, u11); });
             break;
         }
         case SOP_UR: {
             const R u00 = T.mats[op.idx].x, u01 = T.mats[op.idx + 1].x, u10 = T.mats[op.idx + 2].x,
                     u11 = T.mats[op.idx + 3].x;
-            switch (op.a) {
-            case 0: reg_ur<0>(a, u00, u01, u10, u11); break;
-            case 1: reg_ur<1>(a, u00, u01, u10, u11); break;
-            case 2: reg_ur<2>(a, u00, u01, u10, u11); break;
-            default: reg_ur<3>(a, u00, u01, u10, u11); break;
-            }
+            on_bit<N>(op.a, [&](auto B) { reg_ur<B.value>(a, u00, u01, u10, u11); });
             break;
         }
         case SOP_UX: {
             const R u00 = T.mats[op.idx].x, u01 = T.mats[op.idx + 1].y, u10 = T.mats[op.idx + 2].y,
                     u11 = T.mats[op.idx + 3].x;
-            switch (op.a) {
-            case 0: reg_ux<0>(a, u00, u01, u10, u11); break;
-            case 1: reg_ux<1>(a, u00, u01, u10, u11); break;
-            case 2: reg_ux<2>(a, u00, u01, u10, u11); break;
-            default: reg_ux<3>(a, u00, u01, u10, u11); break;
-            }
+            on_bit<N>(op.a, [&](auto B) { reg_ux<B.value>(a, u00, u01, u10, u11); });
             break;
         }
         case SOP_URA:
@@ -699,43 +713,38 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
         case SOP_U2: {
             if constexpr (sizeof(C2) == 16) {
                 const double2* M = reinterpret_cast<const double2*>(&T.mats[op.idx]);
-                switch (op.a * 4 + op.src) {
-                case 1: reg_u2<0, 1>(a, M); break;
-                case 2: reg_u2<0, 2>(a, M); break;
-                case 3: reg_u2<0, 3>(a, M); break;
-                case 6: reg_u2<1, 2>(a, M); break;
-                case 7: reg_u2<1, 3>(a, M); break;
-                default: reg_u2<2, 3>(a, M); break;
+                if constexpr (N == 4) {
+                    reg_u2<0, 1>(a, M);
+                } else if constexpr (N == 8) {
+                    switch (op.a * 4 + op.src) {
+                    case 1: reg_u2<0, 1>(a, M); break;
+                    case 2: reg_u2<0, 2>(a, M); break;
+                    default: reg_u2<1, 2>(a, M); break;
+                    }
+                } else {
+                    switch (op.a * 4 + op.src) {
+                    case 1: reg_u2<0, 1>(a, M); break;
+                    case 2: reg_u2<0, 2>(a, M); break;
+                    case 3: reg_u2<0, 3>(a, M); break;
+                    case 6: reg_u2<1, 2>(a, M); break;
+                    case 7: reg_u2<1, 3>(a, M); break;
+                    default: reg_u2<2, 3>(a, M); break;
+                    }
                 }
             }
             break;
         }
         case SOP_H: {
-            switch (op.a) {
-            case 0: reg_h<0>(a); break;
-            case 1: reg_h<1>(a); break;
-            case 2: reg_h<2>(a); break;
-            default: reg_h<3>(a); break;
-            }
+            on_bit<N>(op.a, [&](auto B) { reg_h<B.value>(a); });
             break;
         }
         case SOP_X: {
             const bool go = (t & op.cthr) == op.cthr && (op.ccos == 0 || (cbase & op.ccos) == op.ccos);
             if (op.cthr == 0) {  // warp-uniform condition: branch
                 if (!go) break;
-                switch (op.a) {
-                case 0: reg_x<0>(a, op.creg); break;
-                case 1: reg_x<1>(a, op.creg); break;
-                case 2: reg_x<2>(a, op.creg); break;
-                default: reg_x<3>(a, op.creg); break;
-                }
+                on_bit<N>(op.a, [&](auto B) { reg_x<B.value>(a, op.creg); });
             } else {
-                switch (op.a) {
-                case 0: reg_xs<0>(a, op.creg, go); break;
-                case 1: reg_xs<1>(a, op.creg, go); break;
-                case 2: reg_xs<2>(a, op.creg, go); break;
-                default: reg_xs<3>(a, op.creg, go); break;
-                }
+                on_bit<N>(op.a, [&](auto B) { reg_xs<B.value>(a, op.creg, go); });
             }
             break;
         }
@@ -743,7 +752,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
             if ((t & op.cthr) != op.cthr || (op.ccos != 0 && (cbase & op.ccos) != op.ccos)) break;
             const C2 ph = T.mats[op.idx];
 #pragma unroll
-            for (int j = 0; j < 16; j++)
+            for (int j = 0; j < N; j++)
                 if (((uint32_t)j & op.creg) == op.creg) a[j] = cmul_r(a[j], ph);
             break;
         }
@@ -752,12 +761,12 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
             const bool b = op.src == SRC_THR ? ((t >> op.a) & 1u) : (uint32_t)((cbase >> op.a) & 1ull);
             const C2 d = b ? d1 : d0;
 #pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = cmul_r(a[j], d);
+            for (int j = 0; j < N; j++) a[j] = cmul_r(a[j], d);
             break;
         }
         case SOP_DR: {
 #pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = cmul_r(a[j], T.mats[op.idx + j]);
+            for (int j = 0; j < N; j++) a[j] = cmul_r(a[j], T.mats[op.idx + j]);
             break;
         }
         default:
@@ -770,7 +779,7 @@ __device__ __forceinline__ void run_program(const TileTables<C2>& T, int nops, u
                 const uint32_t x = s0s >> 4;
                 const uint64_t base = cbase ^ D->sl[x & 63u] ^ D->sh[x >> 6];
 #pragma unroll
-                for (int j = 0; j < 16; j++) gst[base ^ D->sr[j]] = a[j];
+                for (int j = 0; j < N; j++) gst[base ^ D->sr[j]] = a[j];
                 return;
             }
         }

@@ -56,6 +56,16 @@ cudaError_t launch_init_product_c128(void* st, int n, const ProductInit& P, cuda
 cudaError_t launch_pass_generic_c128(void* st, int n, const DevPass& p, const DevOp* ops, const void* pool,
                                      int grid, cudaStream_t s);
 int generic_pass_grid(int n, int m, int device);
+// Register-staged programs [p0, p1) of a state of fewer than 12 qubits, in
+// one CTA (k_small.cu), with 2^reg_bits amplitudes per thread. smem_ops:
+// whether any has shared-memory ops. init: 0 the state as it is, 1 |0...0>,
+// 2 the product state PI. sums (complex128, nullable): the amplitude bit sums
+// of the final state, as launch_bitsums writes them. small_prepare once per
+// device first.
+cudaError_t small_prepare(int device);
+cudaError_t launch_small(void* st, int prec, int n, int reg_bits, const BatchProg* progs, int p0, int p1,
+                         const void* blob, const DevOp* sops, const void* pool, bool smem_ops, int init,
+                         const ProductInit& PI, void* sums, cudaStream_t s);
 // Register-staged tile kernel (12-qubit tiles, 256 threads x 16 amplitudes),
 // prec 0: complex128 / FP64, 1: complex64 / FP32. nbuf = 2: one CTA per SM
 // with a prefetched second tile; nbuf = 1: two CTAs per SM with one tile each.

@@ -869,7 +869,7 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
                 if (pp.prog_note.empty()) pp.bprog = bp;
                 else return "complex64 block lowering failed: " + pp.prog_note;
             }
-        } else if (opt.staged) {
+        } else if (opt.staged && (m == KATE_TILE_BITS || opt.small)) {
             auto prog = std::make_shared<PassProg>();
             // Dense two-qubit gates as register ops when asked for; a pass
             // whose program would then not fit the kernel parameter keeps
@@ -910,7 +910,7 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
                     }
                 }
             }
-            if (pp.prog_note.empty()) pp.prog = prog;
+            if (pp.prog_note.empty()) (m == KATE_TILE_BITS ? pp.prog : pp.sprog) = prog;
         }
         plan.passes.push_back(std::move(pp));
         L.phys = nphys;

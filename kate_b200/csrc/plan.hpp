@@ -53,6 +53,7 @@ struct PlanOptions {
     bool staged = true;  // build register-staged programs for the tile kernel
     bool c64 = false;    // complex64 state: passes become dense 5-qubit tensor-core blocks
     int max_gates_per_pass = 96;  // keeps a pass program within the kernel parameter
+    bool small = false;  // states of fewer than 12 qubits: register-staged programs for the one-CTA kernel
     bool dense2_reg = false;  // dense two-qubit gates as register ops (SOP_U2) rather than shared-memory ops
 };
 
@@ -65,6 +66,7 @@ struct PlannedPass {
     std::vector<int> phys_before;  // layout (logical -> physical) when the pass starts
     std::shared_ptr<PassProg> prog;  // register-staged program (tile kernel), if it applies
     std::shared_ptr<BlockProg> bprog;  // complex64 tensor-core block program, if it applies
+    std::shared_ptr<PassProg> sprog;   // program of the one-CTA kernel (states of fewer than 12 qubits)
     std::string prog_note;           // why the generic kernel runs this pass, if it does
 };
 
@@ -115,13 +117,19 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out);
 std::vector<PlannedPass> plan_relayout(int n, const std::vector<int>& phys, const std::vector<int>& target,
                                        const PlanOptions& opt);
 
-// Register-staged program of a pass (12-qubit tiles). Non-register ops are
-// appended to smem_ops (their tables to pool). Returns "" on success.
+// Register-staged program of a pass (12-qubit tiles, or a whole state of
+// fewer qubits: then with 2^small_reg_bits(n) amplitudes per thread and at
+// least small_reg_bits(n) + 1 tile bits, the bits from n on idle).
+// Non-register ops are appended to smem_ops (their tables to pool). Returns
+// "" on success.
 // low_first: the first stage takes no register among tile bits 0..3 while
 // it has ops without them, so that its lanes 0..3 can read HBM in 256-byte
 // runs (no copy-in through the shared tile).
 std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n, std::vector<DevOp>& smem_ops,
                                std::vector<Cx>& pool, PassProg* out, bool dense2 = false, bool low_first = false);
+
+// Register bits of a program for a state of n < 12 qubits in one tile.
+int small_reg_bits(int n);
 
 // Shared-memory round trips of a register-staged program's tile: one per
 // stage boundary, one for a copy-in when the first stage's registers hold a

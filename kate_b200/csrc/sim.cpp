@@ -71,9 +71,49 @@ struct SimImpl {
     bool prod_start = false;    // the run being enqueued starts with jit_fnP and prod_tab
     ProdTab prod_tab{};
     int jit_grid_n = 0;
+    // States of fewer than 12 qubits: every pass's program, run by one CTA in
+    // one launch (BatchProg headers, then the programs).
+    bool small = false;
+    char* d_small = nullptr;
+    int small_start = 1;  // the run being enqueued: 1 from |0...0>, 2 from small_prod
+    ProductInit small_prod{};
+
+    cudaError_t launch_small_range(int p0, int p1, int init, bool sums, cudaStream_t st) {
+        return launch_small(d_state, precision, n, small_reg_bits(n), (const BatchProg*)d_small, p0, p1, d_small, d_sops, d_pool,
+                            !plan.smem_ops.empty(), init, small_prod, sums ? res_sums() : nullptr, st);
+    }
+    // The programs as one device blob. "" or an error.
+    std::string upload_small() {
+        std::vector<char> blob(plan.passes.size() * sizeof(BatchProg));
+        auto put = [&](const void* p, size_t bytes) {
+            blob.resize((blob.size() + 15) & ~size_t(15));
+            const size_t at = blob.size();
+            blob.insert(blob.end(), (const char*)p, (const char*)p + bytes);
+            return (uint64_t)at;
+        };
+        for (size_t i = 0; i < plan.passes.size(); i++) {
+            const PassProg& P = *plan.passes[i].sprog;
+            BatchProg b{};
+            b.m = P.m;
+            b.nops = P.nops;
+            b.nmats = P.nmats;
+            b.nstages = P.nstages;
+            b.sop0 = P.sop0;
+            b.ops_off = put(P.ops, sizeof(SOp) * (size_t)P.nops);
+            b.mats_off = put(P.mats, 16 * (size_t)P.nmats);
+            b.stab_off = put(P.stab, sizeof(P.stab[0]) * (size_t)P.nstages);
+            std::memcpy(blob.data() + i * sizeof(BatchProg), &b, sizeof b);
+        }
+        blob.resize(((blob.size() + 15) & ~size_t(15)) + 16);
+        KCHECK(cudaMalloc(&d_small, blob.size()));
+        KCHECK(cudaMemcpy(d_small, blob.data(), blob.size(), cudaMemcpyHostToDevice));
+        KCHECK(small_prepare(device));
+        return "";
+    }
 
     // Launches pass i of the plan on stream st.
     cudaError_t launch_pass(size_t i, cudaStream_t st) {
+        if (small) return launch_small_range((int)i, (int)i + 1, 0, false, st);
         const PlannedPass& p = plan.passes[i];
         if (p.bprog) return launch_block_c64(d_state, *p.bprog, d_bimg, d_err, block_grid, st);
         if (i == 0 && zero_start && jit_fn0) return jit_launch(jit_fn0, d_state, *p.prog, jit_grid_n, st);
@@ -209,6 +249,15 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
         const char* jv = std::getenv("KATE_JIT");
         impl->opt.dense2_reg = precision == 0 && !(jv && std::atoi(jv) == 0);
     }
+    if (impl->n < KATE_TILE_BITS) {
+        // The whole state is one tile: nothing to remap between passes, and
+        // the one-CTA kernel computes in FP64 for both precisions.
+        impl->opt.small = true;
+        impl->opt.max_gates_per_pass = 64;  // two register bits: up to 40 stages
+        impl->opt.remap = false;
+        impl->opt.c64 = false;
+        impl->opt.dense2_reg = true;
+    }
     // Complex128 passes of 27 qubits and more choose the qubits they move
     // into the low bits by trying every subset, and the gate cap per pass
     // among a few (about 15 ms of planning for a 30-qubit, 1780-gate
@@ -280,6 +329,12 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
     }
     ce = cached_malloc(&impl->d_state, impl->dim() * impl->amp_bytes(), device);
     if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(state)", ce));
+    impl->small = impl->n < KATE_TILE_BITS;
+    for (const auto& p : impl->plan.passes) impl->small = impl->small && p.sprog;
+    if (impl->small) {
+        e = impl->upload_small();
+        if (!e.empty()) return fail(e);
+    }
     impl->grid = generic_pass_grid(impl->n, std::min(impl->opt.max_tile, impl->n), device);
     if (const char* e = std::getenv("KATE_TILE_NBUF")) {
         const int v = std::atoi(e);
@@ -404,6 +459,7 @@ Simulator::~Simulator() {
     cached_free(d_->d_state, d_->device);
     cudaFree(d_->d_ops);
     cudaFree(d_->d_sops);
+    cudaFree(d_->d_small);
     cudaFree(d_->d_pool);
     cudaFree(d_->d_part);
     pinned_give(d_->pinned);
@@ -457,6 +513,11 @@ std::string Simulator::enqueue_init(void* stream, const double* tp) {
             P.v[1][lab][1] = ei * s0;
         }
         S.prod_start = false;
+        if (S.small) {
+            S.small_prod = P;
+            S.small_start = 2;
+            return "";
+        }
         if (S.jit_fnP && !S.hpasses.empty()) {
             // The first pass computes the product state itself (no
             // initialisation pass, and the state is not read).
@@ -467,6 +528,9 @@ std::string Simulator::enqueue_init(void* stream, const double* tp) {
             return "";
         }
         KCHECK(launch_init_product(S.d_state, S.n, P, S.precision, st));
+    } else if (S.small) {
+        S.small_start = 1;
+        return "";
     } else if (S.jit_fn0) {
         // The first pass writes the whole state from |0...0> itself.
         S.zero_start = true;
@@ -488,7 +552,7 @@ std::string Simulator::execute(const double* tp_in, double* tp_out) {
     if (!e.empty()) return e;
     if (!tp_out) return synchronize();
     const char* r = nullptr;
-    e = S.fetch(&r, true);
+    e = S.fetch(&r, !S.small);
     if (e.empty()) S.proba_from_sums((const double*)r, tp_out);
     return e;
 }
@@ -498,8 +562,9 @@ std::string Simulator::enqueue_passes(void* stream, bool sums) {
     cudaStream_t st = (cudaStream_t)stream;
     const bool zs = S.zero_start, ps = S.prod_start;
     S.zero_start = S.prod_start = false;
+    if (S.small) KCHECK(S.launch_small_range(0, (int)S.hpasses.size(), S.small_start, sums && S.precision == 0, st));
     if (zs && S.hpasses.empty()) KCHECK(launch_set_basis0(S.d_state, S.dim(), S.precision, st));
-    for (size_t i = 0; i < S.hpasses.size(); i++) {
+    for (size_t i = 0; i < S.hpasses.size() && !S.small; i++) {
         S.zero_start = zs && i == 0;
         S.prod_start = ps && i == 0;
         const cudaError_t ce = S.launch_pass(i, st);
@@ -513,7 +578,7 @@ std::string Simulator::enqueue_passes(void* stream, bool sums) {
         else
             KCHECK(launch_renorm_c64(S.d_state, S.n, S.d_norm, st));
         S.renormed = true;
-    } else if (sums) {
+    } else if (sums && !S.small) {
         KCHECK(launch_bitsums(S.d_state, 0, S.n, 0, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
     }
     S.phys = S.plan.final_phys;
@@ -701,6 +766,7 @@ std::string Simulator::profile_passes(float* ms, float* init_ms) {
 }
 
 int Simulator::launches_per_run() const {
+    if (d_->small) return 1 + (d_->precision == 1 ? 2 : 0);
     return (d_->jit_fn0 ? 0 : 1) + (int)d_->hpasses.size() + (d_->precision == 1 ? 2 : 0);
 }
 
@@ -719,6 +785,7 @@ int Simulator::pass_kernel(int i) const {
     if (i < 0 || i >= (int)S.plan.passes.size()) return -1;
     const PlannedPass& p = S.plan.passes[i];
     if (p.bprog) return 3;
+    if (S.small) return 1;
     if (p.prog && (size_t)i < S.jit_fn.size() && S.jit_fn[i]) return 2;
     if (p.prog) return 1;
     return 0;

@@ -61,9 +61,9 @@ bool diag_factors(const std::vector<Cx>& table, int k, std::vector<Cx>* h) {
 // a matrix with a unit entry in each row (SOP_URA/URB/UXA/UXB), picking the
 // factor of larger magnitude so that |t0|, |t1| <= 1, and applies the
 // product F of the factors once: F multiplies the entries of the pass's
-// first diagonal (DR, D1) or general 2x2 (U) op, or, when the pass has none,
+// first diagonal (DR, D1) or general 2x2 or 4x4 (U, U2) op, or, when the pass has none,
 // the first rewritten op goes back to a general 2x2 carrying F.
-void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats) {
+void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats, int nreg) {
     Cx F(1.0, 0.0);
     int first = -1;
     std::vector<Cx> orig;  // matrix of the first rewritten op
@@ -103,7 +103,7 @@ void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats) {
     }
     if (first < 0) return;
     for (SOp& o : ops) {
-        int cnt = o.kind == SOP_DR ? 16 : o.kind == SOP_D1 ? 2 : o.kind == SOP_U ? 4 : 0;
+        int cnt = o.kind == SOP_DR ? nreg : o.kind == SOP_D1 ? 2 : o.kind == SOP_U ? 4 : o.kind == SOP_U2 ? 16 : 0;
         if (!cnt) continue;
         for (int i = 0; i < cnt; i++) mats[o.idx + i] = mats[o.idx + i] * F;
         return;
@@ -126,6 +126,92 @@ int classify_2x2(const Cx* m) {
     return real ? SOP_UR : rx ? SOP_UX : SOP_U;
 }
 
+// Merges each run of two or more ops of one stage that act on the two register
+// bits alone (whatever their kind) into one dense 4x4 (SOP_U2): programs of
+// two register bits, where an op costs its dispatch, not its arithmetic.
+// One-qubit diagonals on thread or coset bits are scalars of a thread and
+// commute with the run.
+void merge_two_bit_runs(std::vector<SOp>& ops, std::vector<Cx>& mats) {
+    std::vector<SOp> out;
+    std::vector<Cx> nm;
+    std::vector<SOp> run;
+    Cx M[16];
+    auto push = [&](SOp o, const Cx* m, int cnt) {
+        if (cnt) o.idx = (uint16_t)nm.size();
+        nm.insert(nm.end(), m, m + cnt);
+        out.push_back(o);
+    };
+    auto count = [](const SOp& o) {
+        switch (o.kind) {
+        case SOP_U: case SOP_UR: case SOP_UX: case SOP_DR: return 4;
+        case SOP_U2: return 16;
+        case SOP_D1: return 2;
+        case SOP_PH: return 1;
+        default: return 0;
+        }
+    };
+    auto flush = [&]() {
+        if (run.size() == 1) {
+            push(run[0], &mats[run[0].idx], count(run[0]));
+        } else if (run.size() > 1) {
+            SOp o{};
+            o.kind = SOP_U2;
+            o.a = 0;
+            o.src = 1;
+            push(o, M, 16);
+        }
+        run.clear();
+    };
+    for (const SOp& o : ops) {
+        Cx A[16];
+        const Cx* m = count(o) ? &mats[o.idx] : nullptr;
+        bool reg = true;
+        switch (o.kind) {
+        case SOP_U: case SOP_UR: case SOP_UX: case SOP_H: {
+            const double h = 0.7071067811865475;
+            const Cx H[4] = {Cx(h, 0), Cx(h, 0), Cx(h, 0), Cx(-h, 0)};
+            const Cx* u = o.kind == SOP_H ? H : m;
+            for (int r = 0; r < 4; r++)
+                for (int c = 0; c < 4; c++)
+                    if (((r ^ c) & ~(1 << o.a)) == 0) A[4 * r + c] = u[2 * ((r >> o.a) & 1) + ((c >> o.a) & 1)];
+            break;
+        }
+        case SOP_DR:
+            for (int r = 0; r < 4; r++) A[5 * r] = m[r];
+            break;
+        case SOP_U2:
+            for (int i = 0; i < 16; i++) A[i] = m[i];
+            break;
+        case SOP_X:
+            reg = o.cthr == 0 && o.ccos == 0;
+            for (int r = 0; r < 4; r++) A[4 * ((r & o.creg) == o.creg ? r ^ (1 << o.a) : r) + r] = Cx(1.0, 0.0);
+            break;
+        default:
+            reg = false;
+        }
+        if (!reg) {
+            if (o.kind != SOP_D1) flush();
+            push(o, m, count(o));
+            continue;
+        }
+        if (run.empty()) {
+            for (int i = 0; i < 16; i++) M[i] = A[i];
+        } else {
+            Cx P[16];
+            for (int r = 0; r < 4; r++)
+                for (int c = 0; c < 4; c++)
+                    for (int k = 0; k < 4; k++) P[4 * r + c] = P[4 * r + c] + A[4 * r + k] * M[4 * k + c];
+            for (int i = 0; i < 16; i++) M[i] = P[i];
+        }
+        run.push_back(o);
+    }
+    flush();
+    ops.swap(out);
+    mats.swap(nm);
+}
+
+int small_reg_bits(int n) { return n <= 10 ? 2 : 3; }
+
 int prog_round_trips(const PassProg& p) {
     if (p.nstages <= 0) return 0;
     int r = p.nstages - 1;
@@ -142,13 +228,18 @@ int prog_round_trips(const PassProg& p) {
 
 std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n, std::vector<DevOp>& smem_ops,
                                std::vector<Cx>& pool, PassProg* out, bool dense2, bool low_first) {
-    const int m = (int)pass.phys_in.size();
-    if (m != KATE_TILE_BITS) return "register-staged kernel needs 12-qubit tiles";
+    const int mq = (int)pass.phys_in.size();
+    if (mq != KATE_TILE_BITS && (mq != n || n > KATE_TILE_BITS)) return "register-staged kernel needs 12-qubit tiles";
+    // A whole state of fewer qubits in one tile: fewer amplitudes per thread
+    // (2^RB), so that one CTA has more warps (at most 8 thread bits).
+    const bool small = mq < KATE_TILE_BITS;
+    const int RB = small ? small_reg_bits(mq) : 4, NA = 1 << RB;
+    const int m = std::max(mq, RB + 1), nthr = m - RB, nwarp = std::max(0, nthr - 5);
     const std::vector<int>& phys = pass.phys_before;
     const int sop_begin = (int)smem_ops.size();
     auto tile_bit = [&](int q) -> int {
         int p = phys[q];
-        for (int t = 0; t < m; t++)
+        for (int t = 0; t < mq; t++)
             if (pass.phys_in[t] == p) return t;
         return -1;
     };
@@ -313,12 +404,12 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
                 const int i = rdy[k];
                 if (regable(i) && missing(i) == 0) at = k;
             }
-            if (at == rdy.size() && R.size() < 4)
+            if (at == rdy.size() && (int)R.size() < RB)
                 for (size_t k = 0; k < rdy.size() && at == rdy.size(); k++) {
                     const int i = rdy[k];
                     const bool avoided = (L[i].tgt >= 0 && !in_R(L[i].tgt) && ((avoid >> L[i].tgt) & 1u)) ||
                                          (L[i].tgt2 >= 0 && !in_R(L[i].tgt2) && ((avoid >> L[i].tgt2) & 1u));
-                    if (regable(i) && L[i].tgt >= 0 && R.size() + missing(i) <= 4 && !avoided) {
+                    if (regable(i) && L[i].tgt >= 0 && (int)R.size() + missing(i) <= RB && !avoided) {
                         at = k;
                         if (!in_R(L[i].tgt)) R.push_back(L[i].tgt);
                         if (L[i].tgt2 >= 0 && !in_R(L[i].tgt2)) R.push_back(L[i].tgt2);
@@ -334,7 +425,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
     };
     auto pad = [&](std::vector<int>& R, uint32_t avoid) {
         for (int pass2 = 0; pass2 < 2; pass2++)
-            for (int t = 0; t < m && R.size() < 4; t++)
+            for (int t = 0; t < m && (int)R.size() < RB; t++)
                 if ((pass2 == 1 || !((avoid >> t) & 1u)) && std::find(R.begin(), R.end(), t) == R.end())
                     R.push_back(t);
     };
@@ -396,7 +487,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             for (int i = 0; i < 4; i++) lowset |= 1u << out->outsrc[i];
         }
         auto is_low = [&](int t) { return ((lowset >> t) & 1u) != 0; };
-        bool local_in = prev_open && prevW.size() == 3;
+        bool local_in = prev_open && (int)prevW.size() == nwarp;
         for (int t : prevW)
             if (!is_nonR(t) || is_low(t)) local_in = false;
         std::vector<int> Wb;
@@ -409,8 +500,8 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             select(dn, Rn, ln, 0);
             if (!ln.empty()) pad(Rn, 0);
             auto in_Rn = [&](int t) { return std::find(Rn.begin(), Rn.end(), t) != Rn.end(); };
-            for (int pass2 = 0; pass2 < 3 && Wb.size() < 3; pass2++)
-                for (int k = (int)nonR.size() - 1; k >= 0 && Wb.size() < 3; k--) {
+            for (int pass2 = 0; pass2 < 3 && (int)Wb.size() < nwarp; pass2++)
+                for (int k = (int)nonR.size() - 1; k >= 0 && (int)Wb.size() < nwarp; k--) {
                     const int t = nonR[k];
                     if (std::find(Wb.begin(), Wb.end(), t) != Wb.end()) continue;
                     const bool ok = pass2 == 0 ? (!is_low(t) && !in_Rn(t)) : pass2 == 1 ? !is_low(t) : true;
@@ -485,7 +576,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
         std::vector<int> lanes, tb;
         for (int t : nonR)
             if (std::find(Wb.begin(), Wb.end(), t) == Wb.end()) lanes.push_back(t);
-        const bool edge = first_stage || last_stage;
+        const bool edge = !small && (first_stage || last_stage);
         bool low4 = edge;
         for (int t = 0; t < m && low4; t++)
             if (is_low(t) && std::find(lanes.begin(), lanes.end(), t) == lanes.end()) low4 = false;
@@ -527,24 +618,24 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
         auto thrpos = [&](int t) { return (int)(std::find(tb.begin(), tb.end(), t) - tb.begin()); };
         if (out->nstages >= KATE_MAX_STAGES) return "pass program has too many stages";
         const int si = out->nstages++;
-        for (int i = 0; i < 4; i++) out->srb[si][i] = (uint8_t)R[i];
-        for (int i = 0; i < 8; i++) out->stb[si][i] = (uint8_t)tb[i];
+        for (int i = 0; i < RB; i++) out->srb[si][i] = (uint8_t)R[i];
+        for (int i = 0; i < nthr; i++) out->stb[si][i] = (uint8_t)tb[i];
         uint16_t* stab = out->stab[si];
         auto swz = [](uint32_t i) { return i ^ (((i >> 3) ^ (i >> 6) ^ (i >> 9)) & 7u); };
         for (int v = 0; v < 16; v++) {
             uint32_t lo = 0, hi = 0;
             for (int i = 0; i < 4; i++) {
-                if ((v >> i) & 1) lo |= 1u << tb[i];
-                if ((v >> i) & 1) hi |= 1u << tb[4 + i];
+                if (((v >> i) & 1) && i < nthr) lo |= 1u << tb[i];
+                if (((v >> i) & 1) && 4 + i < nthr) hi |= 1u << tb[4 + i];
             }
             stab[v] = (uint16_t)(swz(lo) << 4);
             stab[16 + v] = (uint16_t)(swz(hi) << 4);
         }
-        uint32_t wnat[4];
-        for (int i = 0; i < 4; i++) wnat[i] = swz(1u << R[i]) << 4;
+        uint32_t wnat[4] = {0, 0, 0, 0};
+        for (int i = 0; i < RB; i++) wnat[i] = swz(1u << R[i]) << 4;
         auto W = [&](uint32_t x) {
             uint32_t r = 0;
-            for (int k = 0; k < 4; k++)
+            for (int k = 0; k < RB; k++)
                 if ((x >> k) & 1u) r ^= wnat[k];
             return r;
         };
@@ -559,13 +650,13 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             uint64_t ccos;
         };
         auto compose = [&](const std::vector<int>& seq, uint32_t col[4], std::vector<Lane>& lanes) {
-            for (int i = 0; i < 4; i++) col[i] = 1u << i;
+            for (int i = 0; i < RB; i++) col[i] = 1u << i;
             for (int i : seq) {
                 const LOp& o = L[i];
                 const int B = regpos(o.tgt);
                 if (reg_ctl(o)) {
                     const int C = regpos(__builtin_ctz(o.tctl));
-                    for (int k = 0; k < 4; k++) col[k] ^= ((col[k] >> C) & 1u) << B;
+                    for (int k = 0; k < RB; k++) col[k] ^= ((col[k] >> C) & 1u) << B;
                     for (auto& ln : lanes) ln.u ^= ((ln.u >> C) & 1u) << B;
                 } else {
                     Lane ln{1u << B, 0, o.pctl};
@@ -575,9 +666,9 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
                 }
             }
         };
-        auto apply = [](const uint32_t col[4], uint32_t x) {
+        auto apply = [RB](const uint32_t col[4], uint32_t x) {
             uint32_t r = 0;
-            for (int k = 0; k < 4; k++)
+            for (int k = 0; k < RB; k++)
                 if ((x >> k) & 1u) r ^= col[k];
             return r;
         };
@@ -586,7 +677,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
         std::vector<Lane> plane;
         compose(prefix, pcol, plane);
         uint32_t inv[16];
-        for (uint32_t x = 0; x < 16; x++) inv[apply(pcol, x)] = x;
+        for (uint32_t x = 0; x < (uint32_t)NA; x++) inv[apply(pcol, x)] = x;
         std::vector<SOp> xl;
         for (auto& ln : plane) {
             SOp f{};
@@ -596,7 +687,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             f.idx = (uint16_t)W(inv[ln.u]);
             xl.push_back(f);
         }
-        for (int i = 0; i < 4; i++) stab[32 + i] = (uint16_t)W(inv[1u << i]);
+        for (int i = 0; i < RB; i++) stab[32 + i] = (uint16_t)W(inv[1u << i]);
         // Store fold: register j (natural index j) goes to pi(j).
         uint32_t scol[4];
         std::vector<Lane> slane;
@@ -610,8 +701,8 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             f.idx = (uint16_t)W(ln.u);
             folds.push_back(f);
         }
-        for (int i = 0; i < 4; i++) stab[36 + i] = (uint16_t)W(scol[i]);
-        for (int i = 0; i < 4; i++) stab[40 + i] = (uint16_t)wnat[i];
+        for (int i = 0; i < RB; i++) stab[36 + i] = (uint16_t)W(scol[i]);
+        for (int i = 0; i < RB; i++) stab[40 + i] = (uint16_t)wnat[i];
 
         ops.insert(ops.end(), xl.begin(), xl.end());
         SOp st{};
@@ -627,7 +718,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             for (int t = 0; t < m; t++)
                 if ((o.tctl >> t) & 1u) {
                     int r = regpos(t);
-                    if (r < 4) s.creg |= (uint8_t)(1u << r);
+                    if (r < RB) s.creg |= (uint8_t)(1u << r);
                     else s.cthr |= (uint8_t)(1u << thrpos(t));
                 }
             s.ccos = o.pctl;
@@ -648,7 +739,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             SOp f{};
             f.kind = SOP_DR;
             f.idx = (uint16_t)mats.size();
-            mats.insert(mats.end(), dr, dr + 16);
+            mats.insert(mats.end(), dr, dr + NA);
             ops.push_back(f);
             dr_reset();
         };
@@ -690,7 +781,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             case SOP_PH:
                 ctl(o, s);
                 if (s.cthr == 0 && s.ccos == 0) {
-                    for (int j = 0; j < 16; j++)
+                    for (int j = 0; j < NA; j++)
                         if (((uint32_t)j & s.creg) == s.creg) dr[j] = dr[j] * o.m[0];
                     dr_support |= s.creg ? s.creg : 1u;
                     s.kind = 0;
@@ -702,8 +793,8 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
             case SOP_D1:
                 if (o.dtile >= 0) {
                     int r = regpos(o.dtile);
-                    if (r < 4) {
-                        for (int j = 0; j < 16; j++) dr[j] = dr[j] * o.m[(j >> r) & 1];
+                    if (r < RB) {
+                        for (int j = 0; j < NA; j++) dr[j] = dr[j] * o.m[(j >> r) & 1];
                         dr_support |= 1u << r;
                         s.kind = 0;
                         break;
@@ -728,7 +819,8 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
         dr_flush();
         ops.insert(ops.end(), folds.begin(), folds.end());
     }
-    scale_rotations(ops, mats);
+    if (RB == 2) merge_two_bit_runs(ops, mats);
+    scale_rotations(ops, mats, NA);
     if ((int)ops.size() > KATE_MAX_SOPS || (int)mats.size() > KATE_MAX_MATS)
         return "pass program too large for the kernel parameter";
     out->nops = (int)ops.size();
