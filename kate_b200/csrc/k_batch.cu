@@ -87,11 +87,11 @@ __device__ __forceinline__ ProgView view(const BatchProg& P, const unsigned char
 
 // Dynamic shared memory of the batch kernel: two tiles, then the program
 // tables or, for a tensor-core block task, the block region: the B operand
-// images (1024-byte aligned), the BlockProg, the block tables.
+// images (1024-byte aligned), the BlockProg.
 extern __shared__ __align__(16) unsigned char batch_smem_raw[];
 constexpr uint32_t BLK_IMG = KATE_C64_MAX_BLOCKS * KATE_BLOCK_IMG_BYTES;
 constexpr uint32_t BLK_PROG = (sizeof(BlockProg) + 15) & ~15u;
-constexpr uint32_t BLK_REGION = 1024 + BLK_IMG + BLK_PROG + blk::TAB_BYTES + blk::IO_BYTES;
+constexpr uint32_t BLK_REGION = 1024 + BLK_IMG + BLK_PROG;
 static_assert(sizeof(BlockProg) % 8 == 0, "BlockProg is copied as 8-byte words");
 // Per CTA, for the whole launch (complex64 batches with block programs):
 // the products' mbarrier and its phase, the TMEM columns, the wait flag.
@@ -117,8 +117,6 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     const uint32_t bbase = (rawa + 1023u) & ~1023u;
     unsigned char* g = raw + (bbase - rawa);
     BlockProg& P = *reinterpret_cast<BlockProg*>(g + BLK_IMG);
-    uint16_t* tab = reinterpret_cast<uint16_t*>(g + BLK_IMG + BLK_PROG);
-    uint16_t* iot = reinterpret_cast<uint16_t*>(g + BLK_IMG + BLK_PROG + blk::TAB_BYTES);
     const unsigned char* src = blob + BP.ops_off;
     for (uint32_t i = t; i < sizeof(BlockProg) / 8; i += NT)
         reinterpret_cast<uint64_t*>(&P)[i] = __ldcg(reinterpret_cast<const unsigned long long*>(src) + i);
@@ -129,8 +127,8 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     const bool img_ok = blk::load_images(P.nblocks, [&](int b) { return src + P.bimg[b]; }, bbase,
                                          blk::smem_u32(&blk_mbar_img), phase_img);
     if (!img_ok) *abort_flag = 1;
-    blk::Pass X;
-    blk::setup(P, tab, iot, X);
+    blk::Pass<NT> X;
+    blk::setup(P, X);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -140,11 +138,10 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     if (first) {
         for (uint32_t c = c0; c < c1 && ok; c++) {
             const uint64_t cb = blk::coset_base(P, c);
-            blk::zero_tile(S0, cb == 0);
+            blk::zero_tile<NT>(S0, cb == 0);
             __syncthreads();
-            float2* const SS[1] = {S0};
-            ok = blk::apply_blocks<1>(P, X, tab, SS, bbase, tmem, mbar, phase, abort_flag);
-            if (ok) blk::store_tile<true>(P, X, iot, st, cb, S0);
+            ok = blk::apply_blocks(P, X, S0, bbase, tmem, mbar, phase, abort_flag);
+            if (ok) blk::store_tile<true>(P, X, st, cb, S0);
             __syncthreads();
         }
         if (t == 0) {
@@ -153,7 +150,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
         }
         return ok;
     }
-    blk::load_tile<true>(st, blk::coset_base(P, c0), sb0, X, iot);
+    blk::load_tile<true>(st, blk::coset_base(P, c0), sb0, X);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     uint32_t it = 0;
     for (uint32_t c = c0; c < c1; c++, it++) {
@@ -161,16 +158,15 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
         float2* S = S0 + cur * TS;
         // The other buffer was last read by the previous tile's write-back,
         // closed by the barrier at the end of that iteration.
-        if (c + 1 < c1) blk::load_tile<true>(st, blk::coset_base(P, c + 1), sb0 + (cur ^ 1u) * blk::S_BYTES, X, iot);
+        if (c + 1 < c1) blk::load_tile<true>(st, blk::coset_base(P, c + 1), sb0 + (cur ^ 1u) * blk::S_BYTES, X);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");
         __syncthreads();
-        float2* const SS[1] = {S};
-        if (!blk::apply_blocks<1>(P, X, tab, SS, bbase, tmem, mbar, phase, abort_flag)) {
+        if (!blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag)) {
             ok = false;
             break;
         }
-        blk::store_tile<true>(P, X, iot, st, blk::coset_base(P, c), S);
+        blk::store_tile<true>(P, X, st, blk::coset_base(P, c), S);
         __syncthreads();
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");

@@ -2,20 +2,25 @@
 // pass kernel (k_block_c64.cu) and the batch kernel's block tasks
 // (k_batch.cu). A pass applies up to KATE_C64_MAX_BLOCKS dense 5-qubit blocks
 // (BlockProg, device_types.h) to 4096-amplitude coset tiles staged in shared
-// memory; per block:
+// memory. A group of G threads works on a tile (128 in the simulator's pass
+// kernel, two groups per CTA; the whole CTA, 256, in the batch kernel, whose
+// tasks can be a single tile); per block:
 //   1. every thread builds its part of the MMA A operand from the staging
-//      tile: row r = t & 127 (the values of the 7 non-block tile bits), K
-//      half h = t >> 7 (the 16 block indices 16h..16h+15, re/im interleaved),
-//      as a BF16 hi part and the BF16 remainder (lo), and writes it to TMEM
-//      (tcgen05.st; the A operand of tcgen05.mma may live in TMEM: lane r,
-//      one 32-bit column per re/im pair);
+//      tile: row r = t & 127 (the values of the 7 non-block tile bits), all
+//      32 block indices or (G = 256) the 16 of K half t >> 7, re/im
+//      interleaved, as a BF16 hi part and the BF16 remainder (lo), and writes
+//      it to TMEM (tcgen05.st; the A operand of tcgen05.mma may live in TMEM:
+//      lane r, one 32-bit column per re/im pair);
 //   2. one elected thread issues 4 K-steps x 3 products (A_hi.B_hi,
 //      A_hi.B_lo, A_lo.B_hi; M = 128, N = 64, K = 16; A from TMEM, B from
 //      shared memory) into one TMEM accumulator and commits to an mbarrier;
-//   3. every thread reads its row's 32 results back from TMEM and writes
-//      them to the staging tile at the amplitudes' tile positions.
+//   3. every thread reads its row's results back from TMEM and writes them
+//      to the staging tile at the amplitudes' tile positions.
 // Then the tile is written back with the pass's remap permutation (16-byte
-// stores of amplitude pairs). All waits are bounded.
+// stores of amplitude pairs). All waits are bounded. Staging offsets are
+// linear over GF(2) in the index, so every one is a per-thread base XOR a
+// combination of a few values that are the same for all threads (one
+// three-input XOR per access).
 //
 // Accuracy: hi + lo keeps ~16 bits of each FP32 operand and the dropped
 // lo.lo product is ~2^-16 relative, so one block's relative error is about
@@ -39,12 +44,6 @@ constexpr uint32_t S_BYTES = TS * 8;  // one staging tile (float2)
 constexpr uint32_t TMEM_COLS = 128;
 constexpr uint32_t TM_AHI = 64, TM_ALO = 96;
 constexpr long WAIT_LIMIT = 1L << 24;
-// Per-pass tables in shared memory: per block the swizzled tile offset of
-// each block index (32 entries), then 8 swizzled copy offsets P(j << 9), 8
-// write-back offsets P(oH[j]) and P(o1).
-constexpr uint32_t TAB_BYTES = KATE_C64_MAX_BLOCKS * 32 * 2;
-constexpr uint32_t IO_BYTES = 32 * 2;
-
 // The pass's staging-tile swizzle (BlockProg::smask, chosen on the host):
 // element e sits at e ^ sum_k parity(e & f[k]) << k. Linear over GF(2), so
 // offsets of XOR-combined indices XOR.
@@ -162,74 +161,93 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
     }
 }
 
-// A pass's per-thread addressing, built by setup() from a BlockProg.
-struct Pass {
-    uint32_t rsa[KATE_C64_MAX_BLOCKS], rsr[KATE_C64_MAX_BLOCKS];  // swizzled A row / TMEM row offsets
-    uint64_t dT, dH[8];  // global offsets of this thread's 8 amplitude pairs within a coset
-    uint32_t cp_base, wb_base;
-    bool pairs;          // amplitude pairs stay in one 16-byte staging slot
+// Barrier of the G threads that work on one tile: the CTA, or named barrier
+// 1 + (the group's index).
+template <int G>
+__device__ __forceinline__ void group_bar() {
+    if constexpr (G == NT) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / G), "n"(G) : "memory");
+}
+
+// Combinations of four basis values: combo(c, j) = XOR of the c's of the set
+// bits of j, of which v[] holds those of bits 0, 1 and of bits 2, 3.
+struct Combo4 {
+    uint32_t v[6];  // b0, b1, b0 ^ b1, b2, b3, b2 ^ b3
+    __device__ __forceinline__ void set(uint32_t b0, uint32_t b1, uint32_t b2, uint32_t b3) {
+        v[0] = b0, v[1] = b1, v[2] = b0 ^ b1, v[3] = b2, v[4] = b3, v[5] = b2 ^ b3;
+    }
+    __device__ __forceinline__ uint32_t at(uint32_t base, int j) const {  // j a compile-time constant
+        const uint32_t lo = (j & 3) ? v[(j & 3) - 1] : 0u, hi = (j >> 2) ? v[2 + (j >> 2)] : 0u;
+        return base ^ lo ^ hi;
+    }
 };
 
-// Builds the pass's tables (tab, iot in shared memory) and this thread's
-// addressing. The caller places a barrier before the tables are read.
-__device__ __forceinline__ void setup(const BlockProg& P, uint16_t* tab, uint16_t* iot, Pass& X) {
-    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31;
+// A pass's addressing for one thread of a G-thread group, built by setup()
+// from a BlockProg. Copy j of thread t moves the amplitude pair e, e + 1 with
+// e = 2t + 2G j (tile bit 0 is physical bit 0).
+template <int G>
+struct Pass {
+    static constexpr int JB = G == 128 ? 4 : 3;  // bits of j
+    static constexpr int NJ = 1 << JB;
+    uint32_t row[KATE_C64_MAX_BLOCKS];   // swizzled offset of this thread's A row
+    Combo4 blk[KATE_C64_MAX_BLOCKS];     // of block-index bits 0..3
+    uint32_t blk4[KATE_C64_MAX_BLOCKS];  // of block-index bit 4
+    uint64_t dT, dB[4];                  // global offsets of t and of each bit of j within a coset
+    uint32_t cp_base, wb_base, o1;       // staging offsets: copy-in, write-back, write-back's second amplitude
+    Combo4 cp, wb;                       // of the bits of j
+    bool pairs;                          // amplitude pairs stay in one 16-byte staging slot
+    __device__ __forceinline__ uint64_t dH(int j) const {
+        uint64_t d = 0;
+#pragma unroll
+        for (int i = 0; i < JB; i++)
+            if ((j >> i) & 1) d += dB[i];
+        return d;
+    }
+};
+
+template <int G>
+__device__ __forceinline__ void setup(const BlockProg& P, Pass<G>& X) {
+    constexpr int JB = Pass<G>::JB, TBITS = TB - 1 - JB;
+    const uint32_t t = threadIdx.x & (uint32_t)(G - 1);
     const Swz sswz{P.smask[0], P.smask[1], P.smask[2], P.smask[3]};
     X.pairs = P.smask[0] == 0;
 #pragma unroll
     for (int blk = 0; blk < KATE_C64_MAX_BLOCKS; blk++) {
-        X.rsa[blk] = X.rsr[blk] = 0;
+        X.row[blk] = X.blk4[blk] = 0;
+        X.blk[blk].set(0, 0, 0, 0);
         if (blk >= P.nblocks) continue;
         uint32_t bmask = 0;
         for (int i = 0; i < 5; i++) bmask |= 1u << P.btb[blk][i];
-        const uint32_t ra = t & 127u, rr = (warp & 3u) * 32u + lane;
-        uint32_t da = 0, dr = 0;
+        const uint32_t r = t & 127u;  // TMEM lane 32 (warp & 3) + lane
+        uint32_t d = 0;
         for (int i = 0, q = 0; i < TB; i++)
-            if (!((bmask >> i) & 1u)) {
-                da |= ((ra >> q) & 1u) << i;
-                dr |= ((rr >> q) & 1u) << i;
-                q++;
-            }
-        X.rsa[blk] = sswz(da);
-        X.rsr[blk] = sswz(dr);
-        if (t < 32) {
-            uint32_t idx = 0;
-            for (int i = 0; i < 5; i++) idx |= ((t >> i) & 1u) << P.btb[blk][i];
-            tab[blk * 32 + t] = (uint16_t)sswz(idx);
-        }
+            if (!((bmask >> i) & 1u)) d |= ((r >> q++) & 1u) << i;
+        X.row[blk] = sswz(d);
+        X.blk[blk].set(sswz(1u << P.btb[blk][0]), sswz(1u << P.btb[blk][1]), sswz(1u << P.btb[blk][2]),
+                       sswz(1u << P.btb[blk][3]));
+        X.blk4[blk] = sswz(1u << P.btb[blk][4]);
     }
-    // Copy j of thread t moves the amplitude pair e, e + 1 with e = 2t + 512 j
-    // (tile bit 0 is physical bit 0): global offset dT + dH[j]; on write-back
-    // the pair reads the tile at pT | oH[j] and (pT | oH[j]) | o1.
     uint64_t dT = 0;
     uint32_t pT = 0;
-    for (int i = 0; i < 8; i++) {
+    for (int i = 0; i < TBITS; i++) {
         dT |= (uint64_t)((t >> i) & 1u) << P.tphys[i + 1];
         pT |= ((t >> i) & 1u) << P.outsrc[i + 1];
     }
     X.dT = dT;
-    uint32_t oH[8];
+    uint32_t c[4] = {0, 0, 0, 0}, w[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int j = 0; j < 8; j++) {
-        uint64_t g = 0;
-        uint32_t o = 0;
-        for (int i = 0; i < 3; i++)
-            if ((j >> i) & 1) {
-                g |= 1ull << P.tphys[9 + i];
-                o |= 1u << P.outsrc[9 + i];
-            }
-        X.dH[j] = g;
-        oH[j] = o;
+    for (int i = 0; i < 4; i++) {
+        X.dB[i] = 0;
+        if (i >= JB) continue;
+        X.dB[i] = 1ull << P.tphys[1 + TBITS + i];
+        c[i] = sswz(2u * (uint32_t)G << i);
+        w[i] = sswz(1u << P.outsrc[1 + TBITS + i]);
     }
-    const uint32_t o1 = 1u << P.outsrc[0];
-    if (t < 8) {
-        iot[t] = (uint16_t)sswz((uint32_t)t << 9);
-        iot[8 + t] = (uint16_t)sswz(oH[t]);
-    } else if (t == 8) {
-        iot[16] = (uint16_t)sswz(o1);
-    }
-    X.cp_base = sswz(2u * t);  // copy-in: element 2t + 512 j at cp_base ^ iot[j]
-    X.wb_base = sswz(pT);      // write-back: output pair j reads wb_base ^ iot[8 + j]
+    X.cp.set(c[0], c[1], c[2], c[3]);
+    X.wb.set(w[0], w[1], w[2], w[3]);
+    X.cp_base = sswz(2u * t);
+    X.wb_base = sswz(pT);
+    X.o1 = sswz(1u << P.outsrc[0]);
 }
 
 __device__ __forceinline__ uint64_t coset_base(const BlockProg& P, uint64_t c) {
@@ -244,21 +262,20 @@ __device__ __forceinline__ uint64_t coset_base(const BlockProg& P, uint64_t c) {
 // other SMs earlier in the same launch, so an unpaired swizzle's 8-byte
 // copies (which cp.async can only route through L1) become L2 loads and
 // shared stores, visible after the caller's barrier.
-template <bool L2ONLY>
-__device__ __forceinline__ void load_tile(const float2* st, uint64_t cb, uint32_t sb, const Pass& X,
-                                          const uint16_t* iot) {
+template <bool L2ONLY, int G>
+__device__ __forceinline__ void load_tile(const float2* st, uint64_t cb, uint32_t sb, const Pass<G>& X) {
     const float2* src = st + cb + X.dT;
     if (X.pairs) {
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t d = sb + (X.cp_base ^ iot[j]) * 8u;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + X.dH[j]) : "memory");
+        for (int j = 0; j < Pass<G>::NJ; j++) {
+            const uint32_t d = sb + X.cp.at(X.cp_base, j) * 8u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src + X.dH(j)) : "memory");
         }
     } else if (L2ONLY) {
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t e0 = X.cp_base ^ iot[j];
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + X.dH[j]));
+#pragma unroll 8
+        for (int j = 0; j < Pass<G>::NJ; j++) {
+            const uint32_t e0 = X.cp.at(X.cp_base, j);
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + X.dH(j)));
             asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sb + e0 * 8u), "f"(v.x), "f"(v.y) : "memory");
             asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sb + (e0 ^ 1u) * 8u), "f"(v.z), "f"(v.w)
                          : "memory");
@@ -266,12 +283,12 @@ __device__ __forceinline__ void load_tile(const float2* st, uint64_t cb, uint32_
     } else {
         // The pair's two amplitudes land in different 8-byte slots.
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t e0 = X.cp_base ^ iot[j];
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sb + e0 * 8u), "l"(src + X.dH[j])
+        for (int j = 0; j < Pass<G>::NJ; j++) {
+            const uint32_t e0 = X.cp.at(X.cp_base, j);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sb + e0 * 8u), "l"(src + X.dH(j))
                          : "memory");
             asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sb + (e0 ^ 1u) * 8u),
-                         "l"(src + X.dH[j] + 1)
+                         "l"(src + X.dH(j) + 1)
                          : "memory");
         }
     }
@@ -280,40 +297,38 @@ __device__ __forceinline__ void load_tile(const float2* st, uint64_t cb, uint32_
 // Fills the staging tile with the tile of |0...0>: zeros, and 1 at element
 // 0 when `one` (coset 0; element 0 sits at staging offset 0 since the
 // swizzle is linear).
+template <int G>
 __device__ __forceinline__ void zero_tile(float2* S, bool one) {
+    const uint32_t t = threadIdx.x & (uint32_t)(G - 1);
     float4* s4 = reinterpret_cast<float4*>(S);
-    for (uint32_t i = threadIdx.x; i < (uint32_t)TS / 2; i += NT) s4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncthreads();
-    if (one && threadIdx.x == 0) S[0] = make_float2(1.f, 0.f);
+    for (uint32_t i = t; i < (uint32_t)TS / 2; i += G) s4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    group_bar<G>();
+    if (one && t == 0) S[0] = make_float2(1.f, 0.f);
 }
 
-// Applies the pass's blocks to NTL staging tiles S[0..NTL) in lock-step
-// (each copy complete and visible to every thread). Tile i uses the 128 TMEM
-// columns from tmem + 128 i (accumulator, then the A parts). Per block: the
-// A operands of every tile, one barrier, one batch of products for all
-// tiles behind one mbarrier, the read-backs, one barrier; two tiles halve the
-// barriers and product round trips per tile. B images at shared address
-// bimg (block b at bimg + b * KATE_BLOCK_IMG_BYTES, 1024-byte aligned).
-// Returns false when a product wait gave up (after every thread has left
-// the block loop).
-template <int NTL>
-__device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass& X, const uint16_t* tab,
-                                             float2* const (&S)[NTL], uint32_t bimg, uint32_t tmem, uint32_t mbar,
-                                             uint32_t& phase, int* abort_flag) {
-    const uint32_t t = threadIdx.x, warp = t >> 5;
+// Applies the pass's blocks to the staging tile S (its copy complete and
+// visible to every thread of the group), in the 128 TMEM columns from tmem
+// (accumulator, then the A parts). B images at shared address bimg (block b
+// at bimg + b * KATE_BLOCK_IMG_BYTES, 1024-byte aligned). Returns false when
+// a product wait gave up (after every thread of the group has left the block
+// loop).
+template <int G>
+__device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& X, float2* S, uint32_t bimg,
+                                             uint32_t tmem, uint32_t mbar, uint32_t& phase, int* abort_flag) {
+    const uint32_t t = threadIdx.x & (uint32_t)(G - 1);
+    const uint32_t lanes = tmem + (((threadIdx.x >> 5) & 3u) << 21);  // this warp's 32 lanes
+    constexpr uint32_t NH = NT / G;                                   // K halves per thread
     for (int blk = 0; blk < P.nblocks; blk++) {
-        const uint16_t* tb = tab + blk * 32;
-        const uint32_t ra_sw = blk == 0 ? X.rsa[0] : X.rsa[KATE_C64_MAX_BLOCKS - 1];
-        const uint32_t rr_sw = blk == 0 ? X.rsr[0] : X.rsr[KATE_C64_MAX_BLOCKS - 1];
-        const bool wide = P.btb[blk][0] == 0 && X.pairs;  // block index bits 0 = tile bit 0: 16-byte pairs
-        // 1. A operands (hi, lo) from the staging tiles into TMEM. Thread t:
-        //    row r = t & 127 (TMEM lane 32 (warp & 3) + lane), K half
-        //    h = t >> 7 (block indices 16h..16h+15: TMEM columns 16h..16h+15
-        //    of the A parts, one re/im pair per column).
+        const Combo4 C = blk == 0 ? X.blk[0] : X.blk[KATE_C64_MAX_BLOCKS - 1];
+        const uint32_t row = blk == 0 ? X.row[0] : X.row[KATE_C64_MAX_BLOCKS - 1];
+        const uint32_t b4 = blk == 0 ? X.blk4[0] : X.blk4[KATE_C64_MAX_BLOCKS - 1];
+        const bool wide = P.btb[blk][0] == 0 && X.pairs;  // block index bit 0 = tile bit 0: 16-byte pairs
+        // 1. A operands (hi, lo) from the staging tile into TMEM: block
+        //    indices 16h..16h+15 are TMEM columns 16h..16h+15 of the A parts.
 #pragma unroll
-        for (int ti = 0; ti < NTL; ti++) {
-            const float2* St = S[ti];
-            const uint32_t h = t >> 7;
+        for (uint32_t hh = 0; hh < NH; hh++) {
+            const uint32_t h = G == NT ? t >> 7 : hh;
+            const uint32_t base = h ? row ^ b4 : row;
             uint32_t hw[16], lw[16];
             auto split = [&](int e, float2 a) {
                 const uint32_t hp = bf16x2_rn(a.x, a.y);
@@ -324,57 +339,51 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass& X, 
             if (wide) {
 #pragma unroll
                 for (int e = 0; e < 16; e += 2) {
-                    const float4 v = *reinterpret_cast<const float4*>(&St[ra_sw ^ tb[h * 16u + (uint32_t)e]]);
+                    const float4 v = *reinterpret_cast<const float4*>(&S[C.at(base, e)]);
                     split(e, make_float2(v.x, v.y));
                     split(e + 1, make_float2(v.z, v.w));
                 }
             } else {
 #pragma unroll
-                for (int e = 0; e < 16; e++) split(e, St[ra_sw ^ tb[h * 16u + (uint32_t)e]]);
+                for (int e = 0; e < 16; e++) split(e, S[C.at(base, e)]);
             }
-            const uint32_t lane_base = tmem + (uint32_t)ti * 128u + (((warp & 3u) * 32u) << 16) + h * 16u;
-            tmem_st16(lane_base + TM_AHI, hw);
-            tmem_st16(lane_base + TM_ALO, lw);
+            tmem_st16(lanes + TM_AHI + h * 16u, hw);
+            tmem_st16(lanes + TM_ALO + h * 16u, lw);
         }
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
-        // 2. Tensor-core products into TMEM, every tile behind one commit.
+        group_bar<G>();
+        // 2. Tensor-core products into TMEM.
         if (t == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t bb = bimg + (uint32_t)blk * KATE_BLOCK_IMG_BYTES;
 #pragma unroll
-            for (int ti = 0; ti < NTL; ti++) {
-                const uint32_t tm = tmem + (uint32_t)ti * 128u;
-#pragma unroll 1
-                for (int s = 0; s < 4; s++) {
-                    const uint32_t k = (uint32_t)s * 32u;  // K = 16 BF16 = 32 bytes per step (B)
-                    const uint32_t kc = (uint32_t)s * 8u;  // K = 16 BF16 = 8 TMEM columns per step (A)
-                    const uint64_t b_hi = sw128_desc(bb + k), b_lo = sw128_desc(bb + KATE_BLOCK_IMG_BYTES / 2 + k);
-                    mma_bf16_ts(tm, tm + TM_AHI + kc, b_hi, s > 0 ? 1u : 0u);
-                    mma_bf16_ts(tm, tm + TM_AHI + kc, b_lo, 1u);
-                    mma_bf16_ts(tm, tm + TM_ALO + kc, b_hi, 1u);
-                }
+            for (int s = 0; s < 4; s++) {
+                const uint32_t k = (uint32_t)s * 32u;  // K = 16 BF16 = 32 bytes per step (B)
+                const uint32_t kc = (uint32_t)s * 8u;  // K = 16 BF16 = 8 TMEM columns per step (A)
+                const uint64_t b_hi = sw128_desc(bb + k), b_lo = sw128_desc(bb + KATE_BLOCK_IMG_BYTES / 2 + k);
+                mma_bf16_ts(tmem, tmem + TM_AHI + kc, b_hi, s > 0 ? 1u : 0u);
+                mma_bf16_ts(tmem, tmem + TM_AHI + kc, b_lo, 1u);
+                mma_bf16_ts(tmem, tmem + TM_ALO + kc, b_hi, 1u);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
                          : "memory");
         }
         // Every thread waits for the products itself (try_wait suspends the
-        // waiting thread), so no CTA barrier sits between the products and
-        // the read-back. A wait that gives up raises the flag; the read-back
+        // waiting thread), so no barrier sits between the products and the
+        // read-back. A wait that gives up raises the flag; the read-back
         // still runs (its values are then unused) so that every thread
         // reaches the barrier below, after which all see the flag.
         if (!mbar_wait(mbar, phase)) *abort_flag = 1;
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        // 3. Results: warp w reads TMEM lanes 32(w&3)..+31 (rows) and columns
-        //    32(w>>2)..+31 (block indices 16(w>>2)..+15) of each tile.
+        // 3. Results: row t & 127, block indices 16h..16h+15 in columns
+        //    32h..32h+31 of the accumulator.
 #pragma unroll
-        for (int ti = 0; ti < NTL; ti++) {
-            float2* St = S[ti];
-            const uint32_t sub = warp & 3u, ch = warp >> 2;
+        for (uint32_t hh = 0; hh < NH; hh++) {
+            const uint32_t h = G == NT ? t >> 7 : hh;
+            const uint32_t base = h ? row ^ b4 : row;
             uint32_t d[32];
-            const uint32_t taddr = tmem + (uint32_t)ti * 128u + ((sub * 32u) << 16) + ch * 32u;
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
                 "%13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, "
@@ -384,23 +393,22 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass& X, 
                   "=r"(d[15]), "=r"(d[16]), "=r"(d[17]), "=r"(d[18]), "=r"(d[19]), "=r"(d[20]), "=r"(d[21]),
                   "=r"(d[22]), "=r"(d[23]), "=r"(d[24]), "=r"(d[25]), "=r"(d[26]), "=r"(d[27]), "=r"(d[28]),
                   "=r"(d[29]), "=r"(d[30]), "=r"(d[31])
-                : "r"(taddr));
+                : "r"(lanes + h * 32u));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
             if (wide) {
 #pragma unroll
                 for (int e = 0; e < 16; e += 2)
-                    *reinterpret_cast<float4*>(&St[rr_sw ^ tb[ch * 16u + (uint32_t)e]]) =
+                    *reinterpret_cast<float4*>(&S[C.at(base, e)]) =
                         make_float4(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]),
                                     __uint_as_float(d[2 * e + 2]), __uint_as_float(d[2 * e + 3]));
             } else {
 #pragma unroll
                 for (int e = 0; e < 16; e++)
-                    St[rr_sw ^ tb[ch * 16u + (uint32_t)e]] =
-                        make_float2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]));
+                    S[C.at(base, e)] = make_float2(__uint_as_float(d[2 * e]), __uint_as_float(d[2 * e + 1]));
             }
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncthreads();
+        group_bar<G>();
         if (*abort_flag) return false;
     }
     return true;
@@ -409,11 +417,10 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass& X, 
 // Writes the staging tile back with the remap permutation, an amplitude pair
 // per store. st_cg: stores that bypass L1 (the state is read by other SMs
 // later in the same launch).
-template <bool CG>
-__device__ __forceinline__ void store_tile(const BlockProg& P, const Pass& X, const uint16_t* iot, float2* st,
-                                           uint64_t cb, const float2* S) {
+template <bool CG, int G>
+__device__ __forceinline__ void store_tile(const BlockProg& P, const Pass<G>& X, float2* st, uint64_t cb,
+                                           const float2* S) {
     float2* dst = st + cb + X.dT;
-    const uint32_t po1 = iot[16];
     auto put = [&](float2* p, float4 v) {
         if (CG) __stcg(reinterpret_cast<float4*>(p), v);
         else *reinterpret_cast<float4*>(p) = v;
@@ -421,15 +428,25 @@ __device__ __forceinline__ void store_tile(const BlockProg& P, const Pass& X, co
     if (P.outsrc[0] == 0 && X.pairs) {
         // Output bit 0 keeps input bit 0: the pair is one 16-byte slot.
 #pragma unroll
-        for (int j = 0; j < 8; j++) put(dst + X.dH[j], *reinterpret_cast<const float4*>(&S[X.wb_base ^ iot[8 + j]]));
+        for (int j = 0; j < Pass<G>::NJ; j++)
+            put(dst + X.dH(j), *reinterpret_cast<const float4*>(&S[X.wb.at(X.wb_base, j)]));
     } else {
 #pragma unroll
-        for (int j = 0; j < 8; j++) {
-            const uint32_t e0 = X.wb_base ^ iot[8 + j];
-            const float2 v0 = S[e0], v1 = S[e0 ^ po1];
-            put(dst + X.dH[j], make_float4(v0.x, v0.y, v1.x, v1.y));
+        for (int j = 0; j < Pass<G>::NJ; j++) {
+            const uint32_t e0 = X.wb.at(X.wb_base, j);
+            const float2 v0 = S[e0], v1 = S[e0 ^ X.o1];
+            put(dst + X.dH(j), make_float4(v0.x, v0.y, v1.x, v1.y));
         }
     }
+}
+
+// Zeros to every amplitude of a coset (a run from |0...0>: cosets other than
+// the first stay zero under any blocks).
+template <int G>
+__device__ __forceinline__ void store_zero(const Pass<G>& X, float2* st, uint64_t cb) {
+    float2* dst = st + cb + X.dT;
+#pragma unroll
+    for (int j = 0; j < Pass<G>::NJ; j++) *reinterpret_cast<float4*>(dst + X.dH(j)) = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 }  // namespace blk

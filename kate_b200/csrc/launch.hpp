@@ -81,9 +81,11 @@ bool tile_ws_applies(const PassProg& prog);
 int tile_ws_grid(int n, int device);
 cudaError_t launch_tile_ws(void* st, const PassProg& prog, int* err, int grid, cudaStream_t s);
 
-// Complex64 pass of 5-qubit dense blocks on the tensor cores. err: device
-// int set to 1 if a bounded wait gave up.
-cudaError_t launch_block_c64(void* st, const BlockProg& prog, const void* bimg, int* err, int grid, cudaStream_t s);
+// Complex64 pass of 5-qubit dense blocks on the tensor cores. from_zero: the
+// input is |0...0> and the state is not read. err: device int set to 1 if a
+// bounded wait gave up.
+cudaError_t launch_block_c64(void* st, const BlockProg& prog, const void* bimg, bool from_zero, int* err, int grid,
+                             cudaStream_t s);
 int block_c64_grid(int n, int device);
 
 // Persistent batch kernel (k_batch.cu). head, done[circuits], zout (large

@@ -115,7 +115,7 @@ struct SimImpl {
     cudaError_t launch_pass(size_t i, cudaStream_t st) {
         if (small) return launch_small_range((int)i, (int)i + 1, 0, false, st);
         const PlannedPass& p = plan.passes[i];
-        if (p.bprog) return launch_block_c64(d_state, *p.bprog, d_bimg, d_err, block_grid, st);
+        if (p.bprog) return launch_block_c64(d_state, *p.bprog, d_bimg, i == 0 && zero_start, d_err, block_grid, st);
         if (i == 0 && zero_start && jit_fn0) return jit_launch(jit_fn0, d_state, *p.prog, jit_grid_n, st);
         if (i == 0 && prod_start && jit_fnP) return jit_launch_prod(jit_fnP, d_state, *p.prog, prod_tab, jit_grid_n, st);
         if (p.prog && i < jit_fn.size() && jit_fn[i]) return jit_launch(jit_fn[i], d_state, *p.prog, jit_grid_n, st);
@@ -124,6 +124,8 @@ struct SimImpl {
         return launch_pass_generic(d_state, precision, hpasses[i], d_ops, d_pool, grid, st);
     }
     int block_grid = 0;
+    // Whether the first pass generates |0...0> itself.
+    bool starts_from_zero() const { return jit_fn0 || (!plan.passes.empty() && plan.passes[0].bprog); }
 
     uint64_t dim() const { return 1ull << n; }
     size_t amp_bytes() const { return precision == 0 ? 16 : 8; }
@@ -531,7 +533,7 @@ std::string Simulator::enqueue_init(void* stream, const double* tp) {
     } else if (S.small) {
         S.small_start = 1;
         return "";
-    } else if (S.jit_fn0) {
+    } else if (S.starts_from_zero()) {
         // The first pass writes the whole state from |0...0> itself.
         S.zero_start = true;
         S.prod_start = false;
@@ -767,7 +769,7 @@ std::string Simulator::profile_passes(float* ms, float* init_ms) {
 
 int Simulator::launches_per_run() const {
     if (d_->small) return 1 + (d_->precision == 1 ? 2 : 0);
-    return (d_->jit_fn0 ? 0 : 1) + (int)d_->hpasses.size() + (d_->precision == 1 ? 2 : 0);
+    return (d_->starts_from_zero() ? 0 : 1) + (int)d_->hpasses.size() + (d_->precision == 1 ? 2 : 0);
 }
 
 std::string Simulator::norm2_before_renorm(double* out) {
