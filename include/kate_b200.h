@@ -370,9 +370,11 @@ KATE_API kate_status kate_proba_state_noalloc(const void* d_state, size_t state_
  * and is reused by the next simulator or batch on that device that it covers
  * (up to 4x its size), which saves the cudaMalloc / cudaFree of the whole
  * state in a loop of Simulator(circuit).execute(). At most one such buffer
- * is held per device; kate_server_create frees it before taking its budget.
- * This call frees it (device -1: on every device), e.g. before handing the
- * memory to another library. */
+ * is held per device, and up to 16 smaller ones (states and workspaces, 128
+ * MiB in all), 8 streams and 1 MiB of pinned host memory per process;
+ * kate_server_create frees them before taking its budget. This call frees
+ * them (device -1: on every device), e.g. before handing the memory to
+ * another library. */
 KATE_API kate_status kate_release_cached_memory(int device);
 
 /* ---- batches of independent circuits ----

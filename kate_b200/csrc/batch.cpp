@@ -74,6 +74,7 @@ std::string pack_circuit(const Program& in, const BatchTune& tune, bool resident
     o.fuse_1q = true;
     o.staged = true;
     o.c64 = false;
+    o.lower_all = false;
     o.max_gates_per_pass = std::max(1, tune.max_gates);
     // Tensor-core block passes for a complex64 state kept in HBM; a plan
     // with any pass the blocks cannot take keeps register-staged programs.

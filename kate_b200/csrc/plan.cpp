@@ -860,7 +860,7 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
             pp.tile.push_back(q);
             pp.out_tile[t] = (int)(std::lower_bound(S.begin(), S.end(), nphys[q]) - S.begin());
         }
-        lower_pass(plan, pp, L.phys, plan.pool);
+        if (opt.lower_all) lower_pass(plan, pp, L.phys, plan.pool);
         pp.phys_before = L.phys;
         if (opt.c64) {
             if (m == KATE_TILE_BITS) {
@@ -912,6 +912,7 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
             }
             if (pp.prog_note.empty()) (m == KATE_TILE_BITS ? pp.prog : pp.sprog) = prog;
         }
+        if (!opt.lower_all && !pp.prog && !pp.sprog && !pp.bprog) lower_pass(plan, pp, L.phys, plan.pool);
         plan.passes.push_back(std::move(pp));
         L.phys = nphys;
         for (int q = 0; q < n; q++) L.inv[L.phys[q]] = q;

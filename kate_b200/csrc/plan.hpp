@@ -50,6 +50,7 @@ struct PlanOptions {
     bool remap_search = false;  // choose those qubits by trying every c-subset of the tile
     bool cap_search = false;    // plan with several gate caps per pass, keep the plan with the fewest passes
     bool fuse_1q = true; // multiply chains of single-qubit ops on one qubit (FP64, host)
+    bool lower_all = true;  // device ops for every pass (false: only for passes the generic kernel runs)
     bool staged = true;  // build register-staged programs for the tile kernel
     bool c64 = false;    // complex64 state: passes become dense 5-qubit tensor-core blocks
     int max_gates_per_pass = 96;  // keeps a pass program within the kernel parameter

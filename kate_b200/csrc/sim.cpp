@@ -39,6 +39,7 @@ struct SimImpl {
     Plan plan;
     PlanOptions opt;
     void* d_state = nullptr;
+    char* d_ws = nullptr;      // the workspace the pointers below lie in
     DevOp* d_ops = nullptr;
     DevOp* d_sops = nullptr;   // shared-memory ops of register-staged programs
     void* d_pool = nullptr;
@@ -82,8 +83,8 @@ struct SimImpl {
         return launch_small(d_state, precision, n, small_reg_bits(n), (const BatchProg*)d_small, p0, p1, d_small, d_sops, d_pool,
                             !plan.smem_ops.empty(), init, small_prod, sums ? res_sums() : nullptr, st);
     }
-    // The programs as one device blob. "" or an error.
-    std::string upload_small() {
+    // The headers and programs as one blob.
+    std::vector<char> small_blob() const {
         std::vector<char> blob(plan.passes.size() * sizeof(BatchProg));
         auto put = [&](const void* p, size_t bytes) {
             blob.resize((blob.size() + 15) & ~size_t(15));
@@ -105,10 +106,7 @@ struct SimImpl {
             std::memcpy(blob.data() + i * sizeof(BatchProg), &b, sizeof b);
         }
         blob.resize(((blob.size() + 15) & ~size_t(15)) + 16);
-        KCHECK(cudaMalloc(&d_small, blob.size()));
-        KCHECK(cudaMemcpy(d_small, blob.data(), blob.size(), cudaMemcpyHostToDevice));
-        KCHECK(small_prepare(device));
-        return "";
+        return blob;
     }
 
     // Launches pass i of the plan on stream st.
@@ -245,6 +243,7 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
         if (!e.empty()) return fail(e);
     }
     impl->opt.c64 = precision == 1;
+    impl->opt.lower_all = false;
     {
         // Dense two-qubit gates as register ops for complex128, where the
         // pass-specialised kernels run them straight-line.
@@ -287,43 +286,56 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
 
     cudaError_t ce = cudaSetDevice(device);
     if (ce != cudaSuccess) return fail(cuda_err("cudaSetDevice", ce));
-    ce = cudaStreamCreateWithFlags(&impl->stream, cudaStreamNonBlocking);
+    ce = stream_take(&impl->stream, device);
     if (ce != cudaSuccess) return fail(cuda_err("cudaStreamCreate", ce));
-    // Upload ops and the matrix pool.
+    // One workspace holds what the kernels read (uploaded in one copy) and
+    // the measurement's partials.
+    std::vector<char> up;
+    auto put = [&](const void* p, size_t bytes) {
+        const size_t at = (up.size() + 255) & ~size_t(255);
+        up.resize(at + std::max<size_t>(bytes, 16));
+        if (p && bytes) std::memcpy(up.data() + at, p, bytes);
+        return at;
+    };
     std::vector<DevOp> ops;
     for (auto& p : impl->plan.passes) {
         impl->hpasses.push_back(to_devpass(impl->n, p, (int)ops.size()));
         ops.insert(ops.end(), p.ops.begin(), p.ops.end());
     }
-    size_t ops_bytes = std::max<size_t>(1, ops.size()) * sizeof(DevOp);
-    size_t pool_bytes = std::max<size_t>(1, impl->plan.pool.size()) * sizeof(Cx);
-    ce = cudaMalloc(&impl->d_ops, ops_bytes);
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(ops)", ce));
-    ce = cudaMalloc(&impl->d_pool, pool_bytes);
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(pool)", ce));
-    ce = cudaMalloc(&impl->d_sops, std::max<size_t>(1, impl->plan.smem_ops.size()) * sizeof(DevOp));
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(smem ops)", ce));
-    if (!impl->plan.smem_ops.empty())
-        cudaMemcpy(impl->d_sops, impl->plan.smem_ops.data(), impl->plan.smem_ops.size() * sizeof(DevOp),
-                   cudaMemcpyHostToDevice);
-    if (!ops.empty()) cudaMemcpy(impl->d_ops, ops.data(), ops.size() * sizeof(DevOp), cudaMemcpyHostToDevice);
-    if (!impl->plan.pool.empty())
-        cudaMemcpy(impl->d_pool, impl->plan.pool.data(), impl->plan.pool.size() * sizeof(Cx), cudaMemcpyHostToDevice);
-    ce = cudaMalloc(&impl->d_bimg, std::max<size_t>(16, impl->plan.bimg.size()));
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(block images)", ce));
-    if (!impl->plan.bimg.empty())
-        cudaMemcpy(impl->d_bimg, impl->plan.bimg.data(), impl->plan.bimg.size(), cudaMemcpyHostToDevice);
-    if (precision == 1) {
-        ce = cudaMalloc(&impl->d_norm, renorm_scratch_bytes());
-        if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(renormalisation)", ce));
-        cudaMemset(impl->d_norm, 0, renorm_scratch_bytes());
+    const size_t o_err = put(nullptr, sizeof(int));
+    const size_t o_norm = precision == 1 ? put(nullptr, renorm_scratch_bytes()) : 0;
+    const size_t o_ops = put(ops.data(), ops.size() * sizeof(DevOp));
+    const size_t o_sops = put(impl->plan.smem_ops.data(), impl->plan.smem_ops.size() * sizeof(DevOp));
+    const size_t o_pool = put(impl->plan.pool.data(), impl->plan.pool.size() * sizeof(Cx));
+    const size_t o_bimg = put(impl->plan.bimg.data(), impl->plan.bimg.size());
+    impl->small = impl->n < KATE_TILE_BITS;
+    for (const auto& p : impl->plan.passes) impl->small = impl->small && p.sprog;
+    size_t o_small = 0;
+    if (impl->small) {
+        const std::vector<char> blob = impl->small_blob();
+        o_small = put(blob.data(), blob.size());
     }
-    ce = cudaMalloc(&impl->d_err, sizeof(int));
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(error flag)", ce));
-    cudaMemset(impl->d_err, 0, sizeof(int));
-    BitSumShape sh = bitsum_shape(impl->n);
-    ce = cudaMalloc(&impl->d_part, (size_t)sh.grid * sh.nout * 2 * sizeof(double));
-    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(partials)", ce));
+    const BitSumShape sh = bitsum_shape(impl->n);
+    const size_t o_part = (up.size() + 255) & ~size_t(255);
+    const size_t part_bytes = sh.grid > 1 ? (size_t)sh.grid * sh.nout * 2 * sizeof(double) : 16;
+    ce = cached_malloc((void**)&impl->d_ws, o_part + part_bytes, device);
+    if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(workspace)", ce));
+    // On the simulator's stream and waited for: a run may be queued on any stream.
+    ce = cudaMemcpyAsync(impl->d_ws, up.data(), up.size(), cudaMemcpyHostToDevice, impl->stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(impl->stream);
+    if (ce != cudaSuccess) return fail(cuda_err("upload", ce));
+    impl->d_err = (int*)(impl->d_ws + o_err);
+    impl->d_norm = precision == 1 ? impl->d_ws + o_norm : nullptr;
+    impl->d_ops = (DevOp*)(impl->d_ws + o_ops);
+    impl->d_sops = (DevOp*)(impl->d_ws + o_sops);
+    impl->d_pool = impl->d_ws + o_pool;
+    impl->d_bimg = impl->d_ws + o_bimg;
+    impl->d_small = impl->d_ws + o_small;
+    impl->d_part = impl->d_ws + o_part;
+    if (impl->small) {
+        ce = small_prepare(device);
+        if (ce != cudaSuccess) return fail(cuda_err("one-CTA kernel", ce));
+    }
     impl->pinned = (char*)pinned_take();
     if (!impl->pinned) {
         ce = cudaMalloc(&impl->d_res, impl->res_bytes());
@@ -331,12 +343,6 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
     }
     ce = cached_malloc(&impl->d_state, impl->dim() * impl->amp_bytes(), device);
     if (ce != cudaSuccess) return fail(cuda_err("cudaMalloc(state)", ce));
-    impl->small = impl->n < KATE_TILE_BITS;
-    for (const auto& p : impl->plan.passes) impl->small = impl->small && p.sprog;
-    if (impl->small) {
-        e = impl->upload_small();
-        if (!e.empty()) return fail(e);
-    }
     impl->grid = generic_pass_grid(impl->n, std::min(impl->opt.max_tile, impl->n), device);
     if (const char* e = std::getenv("KATE_TILE_NBUF")) {
         const int v = std::atoi(e);
@@ -457,20 +463,15 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
 Simulator::~Simulator() {
     if (!d_) return;
     cudaSetDevice(d_->device);
-    if (d_->stream) cudaStreamSynchronize(d_->stream);
-    cached_free(d_->d_state, d_->device);
-    cudaFree(d_->d_ops);
-    cudaFree(d_->d_sops);
-    cudaFree(d_->d_small);
-    cudaFree(d_->d_pool);
-    cudaFree(d_->d_part);
+    // Nothing of this simulator is in use once the device is idle.
+    const bool idle = device_idle();
+    cached_free(d_->d_state, d_->device, idle);
+    cached_free(d_->d_ws, d_->device, idle);
     pinned_give(d_->pinned);
     cudaFree(d_->d_res);
     cudaFree(d_->d_samp);
-    cudaFree(d_->d_bimg);
-    cudaFree(d_->d_err);
-    cudaFree(d_->d_norm);
-    if (d_->stream) cudaStreamDestroy(d_->stream);
+    if (idle) stream_give(d_->stream, d_->device);
+    else if (d_->stream) cudaStreamDestroy(d_->stream);
     delete d_;
 }
 
