@@ -58,15 +58,25 @@ bool diag_factors(const std::vector<Cx>& table, int k, std::vector<Cx>* h) {
 }  // namespace
 
 // Rewrites real and RX-form 2x2 ops whose matrix is a common factor f times
-// a matrix with a unit entry in each row (SOP_URA/URB/UXA/UXB), picking the
-// factor of larger magnitude so that |t0|, |t1| <= 1, and applies the
+// a matrix with a unit entry in each row (SOP_URA/URB/UXA/UXB) and applies the
 // product F of the factors once: F multiplies the entries of the pass's
-// first diagonal (DR, D1) or general 2x2 or 4x4 (U, U2) op, or, when the pass has none,
-// the first rewritten op goes back to a general 2x2 carrying F.
-void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats, int nreg) {
+// first diagonal (DR, D1) or general 2x2 or 4x4 (U, U2) op, or, when the pass
+// has none, the first rewritten op goes back to a general 2x2 carrying F.
+// Which of two possible factors is taken: with `one_form` the diagonal entry
+// a whenever it can be, so that the op kinds, and with them the kernel
+// generated for the pass, do not depend on the angles (a program that runs
+// circuits of one structure with ever new angles compiles its kernels once;
+// with the larger factor, every new set of angles was a new kernel, about a
+// second of compilation). A row (x0 + i t x1) and its factor round like a x0
+// + i b x1 whatever the size of t; only the range counts: |a| >= 2^-30 and
+// 2^-300 for the product of the pass's factors, else the larger one. Without
+// it (complex64 arithmetic, whose range is small) the larger factor, so that
+// |t0|, |t1| <= 1.
+void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats, int nreg, bool one_form) {
     Cx F(1.0, 0.0);
     int first = -1;
     std::vector<Cx> orig;  // matrix of the first rewritten op
+    double bits = 0.0;     // -log2 of the product of the factors' magnitudes
     for (size_t k = 0; k < ops.size(); k++) {
         SOp& o = ops[k];
         if (o.kind != SOP_UR && o.kind != SOP_UX) continue;
@@ -81,7 +91,9 @@ void scale_rotations(std::vector<SOp>& ops, std::vector<Cx>& mats, int nreg) {
         const bool formA = a == d && a != 0.0;
         const bool formB = b != 0.0 && (ux ? c == b : c == -b);
         if (!formA && !formB) continue;
-        const bool useA = formA && (!formB || std::fabs(a) >= std::fabs(b));
+        const double la = formA ? -std::log2(std::fabs(a)) : 0.0;
+        const bool useA = formA && (!formB || std::fabs(a) >= std::fabs(b) || (one_form && la <= 30 && bits + la <= 300));
+        bits += useA ? la : -std::log2(std::fabs(b));
         if (first < 0) {
             first = (int)k;
             orig.assign(m, m + 4);
@@ -820,7 +832,7 @@ std::string build_pass_program(const Plan& plan, const PlannedPass& pass, int n,
         ops.insert(ops.end(), folds.begin(), folds.end());
     }
     if (RB == 2) merge_two_bit_runs(ops, mats);
-    scale_rotations(ops, mats, NA);
+    scale_rotations(ops, mats, NA, dense2 && !small);
     if ((int)ops.size() > KATE_MAX_SOPS || (int)mats.size() > KATE_MAX_MATS)
         return "pass program too large for the kernel parameter";
     out->nops = (int)ops.size();
