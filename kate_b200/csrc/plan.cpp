@@ -605,25 +605,21 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
             }
         }
         for (auto& t : th) t.join();
-        // Estimated time per amplitude (B200 rates, ps): a pass is bound by
-        // HBM (32 B at 6.5 TB/s), FP64 issue (64 per SM-clock, 148 SMs,
-        // 1.9 GHz) or its shared-memory exchanges (32 B per amplitude each,
-        // 128 B per SM-clock); the on-chip terms carry the 1.5x that the
-        // heavy passes measure against them. Passes with shared-memory ops
+        // Estimated time per amplitude (ps): a pass takes the largest of its
+        // HBM time, its FP64 instructions' and its shared-memory round
+        // trips'. The coefficients are a fit to 181 passes measured at 24 to
+        // 30 qubits (layered, SU(4), QulacsBench, ansatz and QFT circuits,
+        // 30-qubit plans at each cap): 7 % off in the mean square, and in the
+        // measured order for the 30-qubit plans (203, 210, 215 and 227 ps for
+        // caps 144, 128, 112 and 96). Passes with shared-memory ops
         // (interpreter) or without a register-staged program (generic
         // kernel) count three and ten HBM passes.
         auto cost = [](const PlannedPass& pp) {
-            const double hbm = 4.92;
+            const double hbm = 4.9;
             if (!pp.prog) return 10 * hbm;
-            double f = 0;
-            int ex = -1;
-            for (int k = 0; k < pp.prog->nops; k++) {
-                const SOp& o = pp.prog->ops[k];
-                if (o.kind == SOP_SMEM) return 3 * hbm;
-                if (o.kind == SOP_STAGE) ex++;
-                f += sop_fp64_per_amp(o);
-            }
-            return std::max(hbm, 1.5 * std::max(0.0556 * f, 0.89 * std::max(ex, 0)));
+            for (int k = 0; k < pp.prog->nops; k++)
+                if (pp.prog->ops[k].kind == SOP_SMEM) return 3 * hbm;
+            return std::max(hbm, std::max(0.07 * prog_fp64_per_amp(*pp.prog), 2.75 + 1.05 * prog_round_trips(*pp.prog)));
         };
         double best = -1;
         int bk = -1;

@@ -224,6 +224,50 @@ void merge_two_bit_runs(std::vector<SOp>& ops, std::vector<Cx>& mats) {
 
 int small_reg_bits(int n) { return n <= 10 ? 2 : 3; }
 
+double prog_fp64_per_amp(const PassProg& p) {
+    double f = 0;
+    bool qs = false, qc = false;
+    uint32_t qb = 0;
+    auto flush = [&](uint32_t bits) {
+        f += 2.0 * __builtin_popcount(qb & bits);
+        qb &= ~bits;
+    };
+    for (int k = 0; k < p.nops; k++) {
+        const SOp& o = p.ops[k];
+        const uint32_t a = 1u << o.a;
+        switch (o.kind) {
+        case SOP_STAGE:
+            flush(15);
+            if (qs) f += 4;
+            qs = false;
+            break;
+        case SOP_U: flush(a), f += 8; break;                       // 2 DMUL + 6 DFMA
+        case SOP_UR: case SOP_UX: flush(a), f += 4; break;         // 2 DMUL + 2 DFMA
+        case SOP_URA: case SOP_URB: case SOP_UXA: case SOP_UXB: flush(a), f += 2; break;  // 2 DFMA
+        case SOP_H: flush(a), f += 3; break;                       // 2 DADD + 2 DMUL + 2 DFMA per pair
+        case SOP_U2: flush(a | (1u << o.src)), f += 16; break;     // 2 DMUL + 14 DFMA
+        case SOP_X: flush(a); break;
+        case SOP_DR: f += 4; break;                                // complex multiply
+        case SOP_D1:
+            f += 4.0 / 16;
+            (o.src == SRC_THR ? qs : qc) = true;
+            break;
+        case SOP_PH:
+            if (__builtin_popcount(o.creg) > 1) {
+                f += 4.0 / (double)(1u << __builtin_popcount(o.creg));
+                break;
+            }
+            f += 4.0 / 16;
+            if (o.creg) qb |= o.creg;
+            else (o.cthr ? qs : qc) = true;
+            break;
+        default: break;
+        }
+    }
+    flush(15);
+    return f + (qs || qc ? 4 : 0);
+}
+
 int prog_round_trips(const PassProg& p) {
     if (p.nstages <= 0) return 0;
     int r = p.nstages - 1;
