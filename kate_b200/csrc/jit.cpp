@@ -76,6 +76,12 @@ static __device__ __forceinline__ double2 mk(double x, double y) { return make_d
 static __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
+static __device__ __forceinline__ void cfma(double2& a, double2 m, double2 x) {
+    a.x = fma(m.x, x.x, a.x);
+    a.x = fma(-m.y, x.y, a.x);
+    a.y = fma(m.x, x.y, a.y);
+    a.y = fma(m.y, x.x, a.y);
+}
 static __device__ __forceinline__ double2 row2(double2 u0, double2 u1, double2 x, double2 y) {
     double2 r;
     r.x = u0.x * x.x;
@@ -181,6 +187,84 @@ struct Gen {
             if ((j >> b) & 1) o << "    a" << j << " = cmul(a" << j << ", qb" << b << ");\n";
         qb[b] = false;
     }
+    // A dense gate on tile bits d.tb, on the shared tile: each thread takes
+    // whole groups of 2^k amplitudes (k <= 4: their outputs replace them row
+    // by row), or, at k = 5, half the rows of one of the 128 groups, all 32
+    // inputs read as they are needed (16 accumulators; 32 inputs would not
+    // fit the registers). The matrix is M.m[mat0..]. Loops where they do: the
+    // 4096 multiply-adds of a 5-qubit gate as straight-line code took NVRTC
+    // seconds, and those of several 3-qubit gates spilled registers (a
+    // 22-qubit compiled ansatz took 702 us, 354 with loops).
+    void smem_dense(const DevOp& d, int mat0) {
+        const int K = d.k, D = 1 << K;
+        std::vector<int> nb;  // the group index's tile bits: three of distinct residue mod 3 first (bank groups)
+        uint32_t gate = 0;
+        for (int i = 0; i < K; i++) gate |= 1u << d.tb[i];
+        bool res[3] = {false, false, false};
+        for (int b = 0; b < TB; b++)
+            if (!((gate >> b) & 1u) && !res[b % 3]) res[b % 3] = true, nb.push_back(b);
+        for (int b = 0; b < TB; b++)
+            if (!((gate >> b) & 1u) && std::find(nb.begin(), nb.end(), b) == nb.end()) nb.push_back(b);
+        auto off = [&](int v) {
+            uint32_t e = 0;
+            for (int i = 0; i < K; i++)
+                if ((v >> i) & 1) e |= 1u << d.tb[i];
+            return hex32(swz(e) << 4);
+        };
+        o << "    { const u32 gb = (u32)0";
+        for (int i = 0; i < std::min(8, (int)nb.size()); i++)
+            o << " ^ ((t & " << hex32(1u << i) << ") ? " << hex32(swz(1u << nb[i]) << 4) << " : 0u)";
+        o << ";\n";
+        auto bits = [&](const char* v, int n) {  // offset of local index v's low n bits
+            std::string e = "0u";
+            for (int i = 0; i < n; i++)
+                e += std::string(" ^ ((") + v + " >> " + std::to_string(i) + " & 1) ? " + off(1 << i) + " : 0u)";
+            return e;
+        };
+        const std::string md = "M.m[" + std::to_string(mat0) + " + ";
+        if (K <= 4) {
+            const int ng = 1 << (4 - K);
+            std::string gj = "0u";
+            for (int i = 0; i < 4 - K; i++)
+                gj += " ^ ((j >> " + std::to_string(i) + " & 1) ? " + hex32(swz(1u << nb[8 + i]) << 4) + " : 0u)";
+            o << "    _Pragma(\"unroll 1\") for (int j = 0; j < " << ng << "; j++) { const u32 ga = gb ^ (" << gj << ");\n";
+            for (int v = 0; v < D; v++) o << "      const double2 x" << v << " = lds(tb + (ga ^ " << off(v) << "));\n";
+            // Four rows at a time: eight independent chains of multiply-adds.
+            // At k = 4 without a loop: the matrix entries are then operands
+            // of the multiply-adds (in a loop, 256 constant loads per thread
+            // added 90 us to a 23-qubit pass of 200).
+            const int ru = std::min(4, D);
+            const bool loop = K < 4;
+            if (loop) o << "      _Pragma(\"unroll 1\") for (int r = 0; r < " << D << "; r += " << ru << ")\n";
+            for (int r0 = 0; r0 < (loop ? 1 : D); r0 += ru) {
+                auto e = [&](int i, int c) {
+                    return loop ? md + "(r + " + std::to_string(i) + ") * " + std::to_string(D) + " + " + std::to_string(c) + "]"
+                                : m(mat0 + (r0 + i) * D + c);
+                };
+                o << "      { double2 ";
+                for (int i = 0; i < ru; i++) o << (i ? ", y" : "y") << i << " = cmul(" << e(i, 0) << ", x0)";
+                o << ";\n";
+                for (int c = 1; c < D; c++)
+                    for (int i = 0; i < ru; i++) o << "        cfma(y" << i << ", " << e(i, c) << ", x" << c << ");\n";
+                o << "        const u32 gr = ga ^ (" << (loop ? bits("r", K) : off(r0)) << ");\n";
+                for (int i = 0; i < ru; i++) o << "        sts(tb + (gr ^ " << off(i) << "), y" << i << ");\n";
+                o << "      }\n";
+            }
+            o << "    }\n";
+        } else {
+            o << "    double2 y0";
+            for (int r = 1; r < 16; r++) o << ", y" << r;
+            o << ";\n    const u32 hb = t < 128 ? 0u : 512u;\n";
+            for (int r = 0; r < 16; r++) o << "    y" << r << " = mk(0.0, 0.0);\n";
+            o << "    _Pragma(\"unroll 1\") for (int c = 0; c < 32; c++) {\n      const double2 x = lds(tb + (gb ^ (" << bits("c", 5)
+              << ")));\n";
+            for (int r = 0; r < 16; r++) o << "      cfma(y" << r << ", " << md << "hb + " << 32 * r << " + c], x);\n";
+            o << "    }\n    __syncthreads();\n    { const u32 ga = gb ^ (t < 128 ? 0u : " << off(16) << ");\n";
+            for (int r = 0; r < 16; r++) o << "      sts(tb + (ga ^ " << off(r) << "), y" << r << ");\n";
+            o << "    }\n";
+        }
+        o << "    }\n";
+    }
     void flush_stage(bool pass_end) {
         for (int b = 0; b < 4; b++) flush_bit(b);
         if (pass_end && qc) {
@@ -208,56 +292,98 @@ bool lanes_ok(const PassProg& P, int st, const uint8_t* pos) {
 
 }  // namespace
 
-bool jit_pass_work(const PassProg& P, double* fp64, double* smem) {
+bool jit_pass_work(const PassProg& P, const DevOp* sops, double* fp64, double* smem) {
     std::string why;
-    if (jit_pass_source(P, &why).empty()) return false;
+    if (jit_pass_source(P, sops, &why).empty()) return false;
     int first = -1, last = -1, exchanges = 0;
+    bool smem_first = false, smem_last = false;
+    double dense = 0.0;
     for (int k = 0; k < P.nops; k++) {
         const SOp& op = P.ops[k];
         if (op.kind == SOP_STAGE) {
             if (first >= 0) exchanges++;
             if (first < 0) first = op.idx;
             last = op.idx;
+            smem_last = false;
+        } else if (op.kind == SOP_SMEM) {
+            // A dense gate reads and writes the tile once more.
+            if (first < 0) smem_first = true;
+            smem_last = true;
+            exchanges++;
+            dense += 4.0 * (double)(1 << sops[op.idx].k);
         }
     }
     Gen g(P);
     double b = 32.0 * exchanges;
-    if (!lanes_ok(P, first, g.in)) b += 32.0;
-    if (!lanes_ok(P, last, g.out)) b += 32.0;
-    *fp64 = prog_fp64_per_amp(P);
+    if (smem_first || !lanes_ok(P, first, g.in)) b += 32.0;
+    if (smem_last || !lanes_ok(P, last, g.out)) b += 32.0;
+    *fp64 = prog_fp64_per_amp(P) + dense;
     *smem = b;
     return true;
 }
 
-std::string jit_pass_source(const PassProg& P, std::string* why, int form, int occ) {
+namespace {
+// Matrix entries of the pass's dense shared-memory ops, in the order they
+// run; -1 when it has an op the generator does not take.
+int smem_mats(const PassProg& P, const DevOp* sops) {
+    int n = 0;
+    for (int k = 0; k < P.nops; k++) {
+        if (P.ops[k].kind != SOP_SMEM) continue;
+        if (!sops) return -1;
+        const DevOp& d = sops[P.ops[k].idx];
+        if (d.kind != OPK_DENSE || d.k < 1 || d.k > 5) return -1;
+        n += 1 << (2 * d.k);
+    }
+    return n;
+}
+}  // namespace
+
+std::vector<double2> jit_pass_mats(const PassProg& P, const DevOp* sops, const Cx* pool) {
+    std::vector<double2> m;
+    for (int i = 0; i < P.nmats; i++) m.push_back(make_double2(P.mats[i][0], P.mats[i][1]));
+    for (int k = 0; k < P.nops; k++) {
+        if (P.ops[k].kind != SOP_SMEM) continue;
+        const DevOp& d = sops[P.ops[k].idx];
+        for (int i = 0; i < 1 << (2 * d.k); i++) m.push_back(make_double2(pool[d.mat + i].re, pool[d.mat + i].im));
+    }
+    if (m.empty()) m.push_back(make_double2(0.0, 0.0));
+    return m;
+}
+
+std::string jit_pass_source(const PassProg& P, const DevOp* sops, std::string* why, int form, int occ) {
     const bool from_zero = form == 1, from_prod = form == 2;
     auto no = [&](const char* w) {
         if (why) *why = w;
         return std::string();
     };
     if (P.m != TB || P.ncb < 0 || P.ncb > 22) return no("tile shape");
+    const int nsm = smem_mats(P, sops);
+    if (nsm < 0) return no("shared-memory op other than a dense gate");
+    if (P.nmats + nsm > kJitMaxMats) return no("matrices too large for the kernel parameters");
     int first = -1, last = -1;
-    bool wide = false;
+    bool smem_first = false, smem_last = false;
     for (int k = 0; k < P.nops; k++) {
         const int kind = P.ops[k].kind;
-        if (kind == SOP_SMEM) return no("shared-memory op");
-        if (kind == SOP_STAGE) {
-            if (first >= 0 && P.ops[k].src != 1) wide = true;
+        if (kind == SOP_SMEM) {
+            if (first < 0) smem_first = true;
+            smem_last = true;
+        } else if (kind == SOP_STAGE) {
             if (first < 0) first = P.ops[k].idx;
             last = P.ops[k].idx;
+            smem_last = false;
         } else if (first < 0 && kind != SOP_XL && kind != SOP_XF) {
             return no("register op before the first stage");
         }
     }
-    if (first < 0) return no("no stage");
+    if (first < 0 && !smem_first) return no("no stage");
+    if (smem_first && form != 0) return no("a first pass that starts with a shared-memory op");
     for (int s = 0; s < P.nstages; s++)
         if (!stage_linear(P, s)) return no("stage table not linear");
     Gen g(P);
     // okL / okS: the first (last) stage's lanes 0..15 address physical bits
     // 0..3, so it reads (writes) HBM directly in 256-byte runs; otherwise the
     // tile is copied in (out) through shared memory in such runs.
-    const bool okL = lanes_ok(P, first, g.in), okS = lanes_ok(P, last, g.out);
-    (void)wide;
+    const bool okL = !smem_first && lanes_ok(P, first, g.in), okS = !smem_last && lanes_ok(P, last, g.out);
     std::ostringstream& o = g.o;
     int wbo[TB];
     for (int i = 0; i < TB; i++) wbo[i] = i;
@@ -276,7 +402,7 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
             wbo[3] = 6 - pick[0] - pick[1] - pick[2];
         }
     }
-    const int nm = std::max(1, (int)P.nmats);
+    const int nm = std::max(1, (int)P.nmats + nsm);
     o << kPreamble;
     o << "struct __align__(16) Mats { double2 m[" << nm << "]; };\n";
     if (from_prod) o << "struct __align__(16) ProdTab { double2 v[2][" << KATE_MAX_QUBITS << "]; };\n";
@@ -291,7 +417,7 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
         if (P.ops[k].kind == SOP_STAGE) used[P.ops[k].idx] = 1;
     for (int s = 0; s < P.nstages; s++)
         if (used[s] && s != first) o << "  const u32 s0_" << s << " = " << g.thr_expr("u32", s, false, nullptr) << ";\n";
-    o << "  const u32 s0_" << first << " = " << g.thr_expr("u32", first, false, nullptr) << ";\n";
+    if (first >= 0) o << "  const u32 s0_" << first << " = " << g.thr_expr("u32", first, false, nullptr) << ";\n";
     if (okL) o << "  const u64 pin = " << g.thr_expr("u64", first, true, g.in) << ";\n";
     // Tile index (bit k = tile bit k, at physical bit tphys[k]) of a
     // physical offset made of tile bits only.
@@ -390,7 +516,25 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
     o << "    u32 lfl = 0, sfl = 0; u64 lflp = 0, sflp = 0;\n";
     if (from_prod) o << "    u32 lflt = 0;\n";
     bool open = false, started = false;
-    int si = -1;
+    int si = -1, smat = P.nmats;
+    // The coset's tile into shared memory.
+    auto copy_in = [&]() {
+        o << "    { const u64 gb = cb ^ cdT;\n";
+        for (int j = 0; j < 16; j++) {
+            uint64_t go = 0;
+            for (int i = 0; i < 4; i++)
+                if ((j >> i) & 1) go |= 1ull << P.tphys[8 + i];
+            o << "      asm volatile(\"cp.async.cg.shared.global [%0], [%1], 16;\" :: \"r\"(tb + (csw ^ "
+              << hex32(swz((uint32_t)j << 8) << 4) << ")), \"l\"(st + (gb ^ " << hex(go) << ")) : \"memory\");\n";
+        }
+        o << "      asm volatile(\"cp.async.commit_group;\\n\\tcp.async.wait_group 0;\" ::: \"memory\");\n";
+        o << "    }\n    __syncthreads();\n";
+    };
+    auto store_regs = [&]() {
+        g.flush_stage(false);
+        for (int j = 0; j < 16; j++)
+            o << "    sts(tb + ((s0_" << si << " ^ sfl) ^ " << hex32(rvec(P, si, 36, j)) << "), a" << j << ");\n";
+    };
     for (int k = 0; k < P.nops; k++) {
         const SOp& op = P.ops[k];
         // Factors pending on the bits this op targets.
@@ -401,11 +545,7 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
         }
         switch (op.kind) {
         case SOP_STAGE: {
-            if (open) {
-                g.flush_stage(false);
-                for (int j = 0; j < 16; j++)
-                    o << "    sts(tb + ((s0_" << si << " ^ sfl) ^ " << hex32(rvec(P, si, 36, j)) << "), a" << j << ");\n";
-            }
+            if (open) store_regs();
             si = op.idx;
             if (!started && from_prod) {
                 if (okL) {
@@ -444,16 +584,7 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
                 o << "    }\n";
                 started = true;
             } else if (!started && !okL) {
-                o << "    { const u64 gb = cb ^ cdT;\n";
-                for (int j = 0; j < 16; j++) {
-                    uint64_t go = 0;
-                    for (int i = 0; i < 4; i++)
-                        if ((j >> i) & 1) go |= 1ull << P.tphys[8 + i];
-                    o << "      asm volatile(\"cp.async.cg.shared.global [%0], [%1], 16;\" :: \"r\"(tb + (csw ^ "
-                      << hex32(swz((uint32_t)j << 8) << 4) << ")), \"l\"(st + (gb ^ " << hex(go) << ")) : \"memory\");\n";
-                }
-                o << "      asm volatile(\"cp.async.commit_group;\\n\\tcp.async.wait_group 0;\" ::: \"memory\");\n";
-                o << "    }\n    __syncthreads();\n";
+                copy_in();
                 o << "    { const u32 sl = s0_" << si << " ^ lfl;\n";
                 for (int j = 0; j < 16; j++)
                     o << "      a" << j << " = lds(tb + (sl ^ " << hex32(rvec(P, si, 32, j)) << "));\n";
@@ -467,7 +598,8 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
                 o << "    }\n";
                 started = true;
             } else {
-                o << (op.src == 1 ? "    __syncwarp();\n" : "    __syncthreads();\n");
+                // After a shared-memory op the tile is in place already.
+                if (open) o << (op.src == 1 ? "    __syncwarp();\n" : "    __syncthreads();\n");
                 o << "    { const u32 sl = s0_" << si << " ^ lfl;\n";
                 for (int j = 0; j < 16; j++)
                     o << "      a" << j << " = lds(tb + (sl ^ " << hex32(rvec(P, si, 32, j)) << "));\n";
@@ -477,6 +609,19 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
             open = true;
             break;
         }
+        case SOP_SMEM:
+            if (!started) {
+                copy_in();
+                started = true;
+            } else if (open) {
+                store_regs();
+                o << "    __syncthreads();\n";
+            }
+            open = false;
+            g.smem_dense(sops[op.idx], smat);
+            smat += 1 << (2 * sops[op.idx].k);
+            o << "    __syncthreads();\n";
+            break;
         case SOP_XF:
             o << "    if (" << g.cond(op.cthr, op.ccos) << ") { sfl ^= " << hex32(op.idx)
               << "; sflp ^= " << hex(slot_phys((uint32_t)op.idx >> 4, g.out)) << "; }\n";
@@ -610,16 +755,19 @@ std::string jit_pass_source(const PassProg& P, std::string* why, int form, int o
             return no("unknown op");
         }
     }
-    g.flush_stage(true);
+    if (smem_last && g.qc) return no("coset factor after the last stage");
+    if (!smem_last) g.flush_stage(true);
     if (okS) {
         o << "    { const u64 b = cb ^ pout ^ sflp;\n";
         for (int j = 0; j < 16; j++)
             o << "      st[b ^ " << hex(slot_phys(rvec(P, si, 36, j) >> 4, g.out)) << "] = a" << j << ";\n";
         o << "    }\n";
     } else {
-        for (int j = 0; j < 16; j++)
-            o << "    sts(tb + ((s0_" << si << " ^ sfl) ^ " << hex32(rvec(P, si, 36, j)) << "), a" << j << ");\n";
-        o << "    __syncthreads();\n    { const u64 gb = cb ^ cdO;\n";
+        if (!smem_last) {
+            store_regs();
+            o << "    __syncthreads();\n";
+        }
+        o << "    { const u64 gb = cb ^ cdO;\n";
         for (int j = 0; j < 16; j++) {
             uint64_t go = 0;
             uint32_t os = 0;
@@ -792,7 +940,7 @@ std::string jit_compile(int device, const std::vector<std::string>& srcs, std::v
     return "";
 }
 
-std::string jit_pass_key(const PassProg& P, int form, int occ) {
+std::string jit_pass_key(const PassProg& P, const DevOp* sops, int form, int occ) {
     std::string k;
     auto put = [&](const void* p, size_t n) { k.append(static_cast<const char*>(p), n); };
     const int32_t head[7] = {P.m, P.ncb, P.nops, P.nmats, P.nstages, form, occ};
@@ -803,6 +951,13 @@ std::string jit_pass_key(const PassProg& P, int form, int occ) {
     const int nops = std::max(0, std::min((int)P.nops, KATE_MAX_SOPS));
     const int nst = std::max(0, std::min((int)P.nstages, KATE_MAX_STAGES));
     put(P.ops, sizeof(SOp) * (size_t)nops);
+    for (int k = 0; k < nops && sops; k++)
+        if (P.ops[k].kind == SOP_SMEM) {
+            const DevOp& d = sops[P.ops[k].idx];
+            put(&d.kind, sizeof d.kind);
+            put(&d.k, sizeof d.k);
+            put(d.tb, sizeof d.tb);
+        }
     put(P.stab, sizeof(P.stab[0]) * (size_t)nst);
     put(P.srb, sizeof(P.srb[0]) * (size_t)nst);
     put(P.stb, sizeof(P.stb[0]) * (size_t)nst);
@@ -844,21 +999,9 @@ int jit_grid(int ncb, int device) {
     return 1 << ncb;  // one coset per CTA
 }
 
-cudaError_t jit_launch_prod(void* fn, void* st, const PassProg& prog, const ProdTab& pt, int grid, cudaStream_t s) {
-    double2 mats[KATE_MAX_MATS];
-    const int nm = std::max(1, (int)prog.nmats);
-    for (int i = 0; i < nm; i++) mats[i] = make_double2(i < prog.nmats ? prog.mats[i][0] : 0.0, i < prog.nmats ? prog.mats[i][1] : 0.0);
-    ProdTab p = pt;
-    void* args[] = {&st, mats, &p};
-    const CUresult r = api().launch((CUfunction)fn, grid, 1, 1, 256, 1, 1, 65536, (CUstream)s, args, nullptr);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
-}
-
-cudaError_t jit_launch(void* fn, void* st, const PassProg& prog, int grid, cudaStream_t s) {
-    double2 mats[KATE_MAX_MATS];
-    const int nm = std::max(1, (int)prog.nmats);
-    for (int i = 0; i < nm; i++) mats[i] = make_double2(i < prog.nmats ? prog.mats[i][0] : 0.0, i < prog.nmats ? prog.mats[i][1] : 0.0);
-    void* args[] = {&st, mats};
+cudaError_t jit_launch(void* fn, void* st, const std::vector<double2>& mats, const ProdTab* pt, int grid,
+                       cudaStream_t s) {
+    void* args[] = {&st, const_cast<double2*>(mats.data()), const_cast<ProdTab*>(pt)};
     const CUresult r = api().launch((CUfunction)fn, grid, 1, 1, 256, 1, 1, 65536, (CUstream)s, args, nullptr);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }

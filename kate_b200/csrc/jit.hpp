@@ -19,13 +19,14 @@
 #include <string>
 #include <vector>
 
+#include "circuit.hpp"
 #include "device_types.h"
 
 namespace kate {
 
 // CUDA source of the kernel for `prog`, or "" (with *why set) when the
-// program has a form the generator does not take (shared-memory ops, a
-// register op before the first stage). from_zero: the pass is the first of
+// program has a form the generator does not take (shared-memory ops other than
+// dense gates, a register op before the first stage). from_zero: the pass is the first of
 // a run from |0...0>; it generates its input instead of loading it (only
 // coset 0 is nonzero; every other coset's output is zero, written without
 // being read), so the run needs no separate initialisation pass.
@@ -36,7 +37,17 @@ namespace kate {
 // v[bit p][p] (coset factor times two 64-entry tile tables), from a second
 // parameter (ProdTab), so no initialisation pass runs and the state is not
 // read.
-std::string jit_pass_source(const PassProg& prog, std::string* why, int form = 0, int occ = 2);
+// sops: the plan's shared-memory ops from prog.sop0 on; dense gates of up to
+// five qubits among them run on the shared tile between the stages (without
+// sops, or with other ops, the generator declines).
+std::string jit_pass_source(const PassProg& prog, const DevOp* sops, std::string* why, int form = 0, int occ = 2);
+
+// Matrix entries a kernel's parameters hold at most (32,764 bytes with the
+// state pointer and a ProdTab).
+constexpr int kJitMaxMats = 1950;
+// The matrices parameter of the kernel: prog's own, then those of its dense
+// shared-memory ops (from `pool`) in the order they run.
+std::vector<double2> jit_pass_mats(const PassProg& prog, const DevOp* sops, const Cx* pool);
 
 // Compiles the sources not yet cached on `device` (in parallel) and returns
 // a kernel handle per source. Returns "" on success.
@@ -46,7 +57,7 @@ std::string jit_compile(int device, const std::vector<std::string>& srcs, std::v
 // the matrix values), with from_zero and occ: a key a few KB long, so a
 // simulator whose passes were compiled before finds their kernels without
 // generating their sources (about 0.2 ms per pass).
-std::string jit_pass_key(const PassProg& prog, int form, int occ);
+std::string jit_pass_key(const PassProg& prog, const DevOp* sops, int form, int occ);
 // The kernel compiled on `device` for a pass key, or null.
 void* jit_find(int device, const std::string& key);
 // Records the kernel of a pass key (from jit_compile).
@@ -58,7 +69,7 @@ void jit_remember(int device, const std::string& key, void* fn);
 // bytes moved (16 B stored and 16 B loaded per amplitude for each stage
 // exchange, for a copy-in through the tile and for a write-back through
 // it). False when the generator does not take the program.
-bool jit_pass_work(const PassProg& prog, double* fp64_per_amp, double* smem_bytes_per_amp);
+bool jit_pass_work(const PassProg& prog, const DevOp* sops, double* fp64_per_amp, double* smem_bytes_per_amp);
 
 // Local memory (register spill) bytes per thread of a compiled kernel; -1
 // when unknown.
@@ -67,14 +78,14 @@ int jit_local_bytes(void* fn);
 // Grid of a pass-specialised kernel for 2^ncb cosets on `device`.
 int jit_grid(int ncb, int device);
 
-// Launches kernel fn (from jit_compile) on the complex128 state st with the
-// matrices of prog.
-cudaError_t jit_launch(void* fn, void* st, const PassProg& prog, int grid, cudaStream_t s);
 // The per-qubit factors of a form-2 kernel: v[b][p] multiplies amplitudes
 // whose physical bit p is b.
 struct ProdTab {
     double2 v[2][KATE_MAX_QUBITS];
 };
-cudaError_t jit_launch_prod(void* fn, void* st, const PassProg& prog, const ProdTab& pt, int grid, cudaStream_t s);
+// Launches kernel fn (from jit_compile) on the complex128 state st with the
+// matrices of jit_pass_mats and, for a form-2 kernel, the factors pt.
+cudaError_t jit_launch(void* fn, void* st, const std::vector<double2>& mats, const ProdTab* pt, int grid,
+                       cudaStream_t s);
 
 }  // namespace kate

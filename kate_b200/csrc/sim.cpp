@@ -66,6 +66,9 @@ struct SimImpl {
     int ws_grid = 0;
     std::vector<char> ws_ok;  // pass i runs on the warp-specialised complex128 tile kernel
     std::vector<void*> jit_fn;  // pass i runs on its pass-specialised kernel (complex128)
+    std::vector<std::vector<double2>> jit_mats;  // its matrices (kernel parameter)
+    // Shared-memory ops of pass i's program.
+    const DevOp* sops_of(size_t i) const { return plan.smem_ops.data() + plan.passes[i].prog->sop0; }
     void* jit_fn0 = nullptr;    // pass 0 generating its input |0...0> (no initialisation pass)
     bool zero_start = false;    // the run being enqueued starts with jit_fn0
     void* jit_fnP = nullptr;    // pass 0 computing a product-state input (no initialisation pass)
@@ -114,9 +117,9 @@ struct SimImpl {
         if (small) return launch_small_range((int)i, (int)i + 1, 0, false, st);
         const PlannedPass& p = plan.passes[i];
         if (p.bprog) return launch_block_c64(d_state, *p.bprog, d_bimg, i == 0 && zero_start, d_err, block_grid, st);
-        if (i == 0 && zero_start && jit_fn0) return jit_launch(jit_fn0, d_state, *p.prog, jit_grid_n, st);
-        if (i == 0 && prod_start && jit_fnP) return jit_launch_prod(jit_fnP, d_state, *p.prog, prod_tab, jit_grid_n, st);
-        if (p.prog && i < jit_fn.size() && jit_fn[i]) return jit_launch(jit_fn[i], d_state, *p.prog, jit_grid_n, st);
+        if (i == 0 && zero_start && jit_fn0) return jit_launch(jit_fn0, d_state, jit_mats[0], nullptr, jit_grid_n, st);
+        if (i == 0 && prod_start && jit_fnP) return jit_launch(jit_fnP, d_state, jit_mats[0], &prod_tab, jit_grid_n, st);
+        if (p.prog && i < jit_fn.size() && jit_fn[i]) return jit_launch(jit_fn[i], d_state, jit_mats[i], nullptr, jit_grid_n, st);
         if (p.prog && i < ws_ok.size() && ws_ok[i]) return launch_tile_ws(d_state, *p.prog, d_err, ws_grid, st);
         if (p.prog) return launch_tile(d_state, precision, *p.prog, d_sops, d_pool, tile_grid, nbuf, st);
         return launch_pass_generic(d_state, precision, hpasses[i], d_ops, d_pool, grid, st);
@@ -372,13 +375,13 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
             std::vector<std::string> keys;
             std::vector<size_t> miss;
             auto want = [&](size_t i, int form, int occ) {
-                std::string key = jit_pass_key(*impl->plan.passes[i].prog, form, occ);
+                std::string key = jit_pass_key(*impl->plan.passes[i].prog, impl->sops_of(i), form, occ);
                 void* f = jit_find(device, key);
                 idx.push_back(i);
                 forms.push_back(form);
                 if (!f) {
                     miss.push_back(fns.size());
-                    todo.push_back(jit_pass_source(*impl->plan.passes[i].prog, nullptr, form, occ));
+                    todo.push_back(jit_pass_source(*impl->plan.passes[i].prog, impl->sops_of(i), nullptr, form, occ));
                 }
                 fns.push_back(f);
                 keys.push_back(std::move(key));
@@ -418,11 +421,12 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
                 // A kernel that spills at three CTAs per SM goes back to two.
                 for (size_t k = 0; k < fns.size(); k++)
                     if (fns[k] && jit_local_bytes(fns[k]) != 0) {
-                        std::string key = jit_pass_key(*impl->plan.passes[idx[k]].prog, forms[k], 2);
+                        std::string key = jit_pass_key(*impl->plan.passes[idx[k]].prog, impl->sops_of(idx[k]), forms[k], 2);
                         void* f = jit_find(device, key);
                         if (!f) {
                             miss.push_back(k);
-                            todo.push_back(jit_pass_source(*impl->plan.passes[idx[k]].prog, nullptr, forms[k], 2));
+                            todo.push_back(jit_pass_source(*impl->plan.passes[idx[k]].prog, impl->sops_of(idx[k]), nullptr,
+                                                           forms[k], 2));
                         }
                         fns[k] = f;
                         keys[k] = std::move(key);
@@ -431,9 +435,14 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
                 if (!je.empty()) return fail("pass kernel compilation: " + je);
             }
             impl->jit_fn.assign(impl->plan.passes.size(), nullptr);
+            impl->jit_mats.resize(impl->plan.passes.size());
             for (size_t k = 0; k < idx.size(); k++) {
                 if (!fns[k]) continue;
-                if (forms[k] == 0) impl->jit_fn[idx[k]] = fns[k];
+                if (forms[k] == 0) {
+                    impl->jit_fn[idx[k]] = fns[k];
+                    impl->jit_mats[idx[k]] = jit_pass_mats(*impl->plan.passes[idx[k]].prog, impl->sops_of(idx[k]),
+                                                           impl->plan.pool.data());
+                }
                 else if (forms[k] == 1) impl->jit_fn0 = fns[k];
                 else impl->jit_fnP = fns[k];
             }
@@ -797,7 +806,7 @@ int Simulator::pass_kernel(int i) const {
 bool Simulator::pass_work(int i, double out[3]) const {
     if (pass_kernel(i) != 2) return false;
     out[0] = 2.0 * 16.0;
-    return jit_pass_work(*d_->plan.passes[i].prog, &out[1], &out[2]);
+    return jit_pass_work(*d_->plan.passes[i].prog, d_->sops_of((size_t)i), &out[1], &out[2]);
 }
 
 std::string Simulator::state_device(void** dptr, int* phys) {
