@@ -412,6 +412,15 @@ std::string jit_pass_source(const PassProg& P, const DevOp* sops, std::string* w
     o << "  extern __shared__ __align__(16) unsigned char smem[];\n";
     o << "  const u32 tb = (u32)__cvta_generic_to_shared(smem);\n";
     o << "  const u32 t = threadIdx.x;\n";
+    // Launched to start before the pass before it has finished (jit_launch):
+    // everything up to the wait below touches no memory but the parameters.
+    // Only short passes (up to 1024 CTAs, 22 qubits) let the next one start
+    // early, which hides 1.5 to 2 us each (20 qubits, 10 passes: 125 -> 110
+    // us), and none with dense two-qubit gates: the instruction costs those
+    // kernels' register allocation more (26-qubit SU(4) passes 5.2 -> 6.3 ms).
+    bool u2 = false;
+    for (int k = 0; k < P.nops; k++) u2 = u2 || P.ops[k].kind == SOP_U2;
+    if (P.ncb <= 10 && !u2) o << "  asm volatile(\"griddepcontrol.launch_dependents;\" ::: \"memory\");\n";
     std::vector<char> used(P.nstages, 0);
     for (int k = 0; k < P.nops; k++)
         if (P.ops[k].kind == SOP_STAGE) used[P.ops[k].idx] = 1;
@@ -470,6 +479,7 @@ std::string jit_pass_source(const PassProg& P, const DevOp* sops, std::string* w
           << ";\n";
         i = j + 1;
     }
+    o << "    asm volatile(\"griddepcontrol.wait;\" ::: \"memory\");\n";
     if (from_zero) {
         // The input is |0...0>: every coset but 0 is zero in and out, so its
         // output is written without being read or computed.
@@ -799,8 +809,7 @@ struct Api {
     CUresult (*set_attr)(CUfunction, CUfunction_attribute, int);
     CUresult (*occupancy)(int*, CUfunction, int, size_t);
     CUresult (*get_attr)(int*, CUfunction_attribute, CUfunction);
-    CUresult (*launch)(CUfunction, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, CUstream,
-                       void**, void**);
+    CUresult (*launch)(const CUlaunchConfig*, CUfunction, void**, void**);
     std::string nvrtc_err, drv_err;
     bool nvrtc_ok = false, drv_ok = false;
 };
@@ -837,7 +846,7 @@ Api& api() {
                    drv("cuFuncSetAttribute", (void**)&a.set_attr) &&
                    drv("cuOccupancyMaxActiveBlocksPerMultiprocessor", (void**)&a.occupancy) &&
                    drv("cuFuncGetAttribute", (void**)&a.get_attr) &&
-                   drv("cuLaunchKernel", (void**)&a.launch);
+                   drv("cuLaunchKernelEx", (void**)&a.launch);
         if (!a.drv_ok) a.drv_err = "CUDA driver entry points unavailable";
     });
     return a;
@@ -1002,7 +1011,18 @@ int jit_grid(int ncb, int device) {
 cudaError_t jit_launch(void* fn, void* st, const std::vector<double2>& mats, const ProdTab* pt, int grid,
                        cudaStream_t s) {
     void* args[] = {&st, const_cast<double2*>(mats.data()), const_cast<ProdTab*>(pt)};
-    const CUresult r = api().launch((CUfunction)fn, grid, 1, 1, 256, 1, 1, 65536, (CUstream)s, args, nullptr);
+    CUlaunchAttribute a{};
+    a.id = CU_LAUNCH_ATTRIBUTE_PROGRAMMATIC_STREAM_SERIALIZATION;
+    a.value.programmaticStreamSerializationAllowed = 1;
+    CUlaunchConfig c{};
+    c.gridDimX = (unsigned)grid;
+    c.gridDimY = c.gridDimZ = c.blockDimY = c.blockDimZ = 1;
+    c.blockDimX = 256;
+    c.sharedMemBytes = 65536;
+    c.hStream = (CUstream)s;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    const CUresult r = api().launch(&c, (CUfunction)fn, args, nullptr);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }
 

@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include "k_block.cuh"
+#include "k_common.cuh"
 #include "launch.hpp"
 
 namespace kate {
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(NT, 2)
     k_block_c64(float2* __restrict__ st, const __grid_constant__ BlockProg P, const uint8_t* __restrict__ bimg,
                 int from_zero, int* __restrict__ err) {
     extern __shared__ uint8_t smem_raw[];
+    let_next_start();
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // 1024-byte aligned operand region
     uint8_t* gbase = smem_raw + (base - raw);
@@ -68,6 +70,7 @@ __global__ void __launch_bounds__(NT, 2)
     float2* S = reinterpret_cast<float2*>(gbase + OFF_S + grp * S_BYTES);
     const uint32_t sb = base + OFF_S + grp * S_BYTES;
     uint32_t phase = 0;
+    wait_for_previous();  // everything above reads only what no pass writes
     for (uint64_t c = (uint64_t)blockIdx.x * NG + grp; c < ncos; c += (uint64_t)gridDim.x * NG) {
         const uint64_t cb = coset_base(P, c);
         if (from_zero) {
@@ -116,8 +119,7 @@ cudaError_t launch_block_c64(void* st, const BlockProg& prog, const void* bimg, 
                              cudaStream_t s) {
     if (prog.m != TB || prog.nblocks < 1 || prog.nblocks > KATE_C64_MAX_BLOCKS) return cudaErrorInvalidValue;
     if (prog.tphys[0] != 0) return cudaErrorInvalidValue;  // amplitude pairs must be contiguous
-    k_block_c64<<<grid, NT, SMEM_BYTES, s>>>((float2*)st, prog, (const uint8_t*)bimg, from_zero, err);
-    return cudaGetLastError();
+    return launch_after(k_block_c64, grid, NT, SMEM_BYTES, s, (float2*)st, prog, (const uint8_t*)bimg, (int)from_zero, err);
 }
 
 }  // namespace kate

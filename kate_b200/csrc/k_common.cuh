@@ -9,6 +9,13 @@ namespace kate {
 #define KATE_SQRT2 1.4142135623730951
 #define KATE_SQRT2INV 0.7071067811865475
 
+// Programmatic dependent launch (launch_after, launch.hpp): a kernel of a
+// chain lets the next one start its prologue once all of its own CTAs run, and
+// waits, before it touches what the one before writes, until that has finished
+// and its writes are visible. Both are no-ops in a plain launch.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Inserts a zero bit at position b of v.
 __device__ __forceinline__ uint32_t ins0(uint32_t v, int b) {
     return ((v >> b) << (b + 1)) | (v & ((1u << b) - 1u));

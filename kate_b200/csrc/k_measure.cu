@@ -107,6 +107,8 @@ __global__ void __launch_bounds__(NT, 3) k_bitsums(S* __restrict__ st, int n, in
                                                    const double* __restrict__ scale, const int* __restrict__ err,
                                                    int* __restrict__ err_out) {
     using A = Acc<V>;
+    let_next_start();
+    wait_for_previous();
     if (err_out && blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;
     constexpr bool F = sizeof(S) == 8;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
@@ -197,6 +199,8 @@ template <typename V>
 __global__ void __launch_bounds__(NT) k_bitsums_finish(const V* __restrict__ part, int g, int first,
                                                        V* __restrict__ out) {
     using A = Acc<V>;
+    let_next_start();
+    wait_for_previous();
     const uint32_t o = blockIdx.x + (uint32_t)first, t = threadIdx.x, ncta = 1u << g;
     const int b = o ? (int)(o - 1) / 2 : 0, one = o ? (int)(o - 1) & 1 : 0;
     const bool cta_bit = o && b >= 12 && b < 12 + g;
@@ -241,6 +245,8 @@ __global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st
                                                    double* __restrict__ out) {
     __shared__ double red[256];
     __shared__ bool last;
+    let_next_start();
+    wait_for_previous();
     const uint32_t t = threadIdx.x;
     const uint64_t stride = (uint64_t)gridDim.x * 256;
     double acc = 0.0;
@@ -296,6 +302,8 @@ __global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st
 // by up to 2^-23.
 __global__ void __launch_bounds__(256) k_scale_c64(float4* __restrict__ st, uint64_t npairs,
                                                    const double* __restrict__ out) {
+    let_next_start();
+    wait_for_previous();
     const double f = out[1];
     const uint64_t stride = (uint64_t)gridDim.x * 256;
     for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < npairs; i += stride) {
@@ -319,8 +327,7 @@ cudaError_t launch_norm_c64(const void* st, int n, void* scratch, cudaStream_t s
     double* out = part + RN_GRID;
     unsigned* count = (unsigned*)(out + 2);
     const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
-    k_norm2_c64<<<grid, 256, 0, s>>>((const float4*)st, npairs, part, count, out);
-    return cudaGetLastError();
+    return launch_after(k_norm2_c64, grid, 256, 0, s, (const float4*)st, npairs, part, count, out);
 }
 
 cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
@@ -328,8 +335,7 @@ cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const uint64_t npairs = (1ull << n) / 2;
     const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
-    k_scale_c64<<<grid, 256, 0, s>>>((float4*)st, npairs, (const double*)scratch + RN_GRID);
-    return cudaGetLastError();
+    return launch_after(k_scale_c64, grid, 256, 0, s, (float4*)st, npairs, (const double*)scratch + RN_GRID);
 }
 
 BitSumShape bitsum_shape(int n) {
@@ -357,11 +363,9 @@ cudaError_t bitsums(S* st, int n, int g, int nr, void* partials, void* out, cons
     if (n >= 12 ? n != 12 + g + nr : g + nr != 0) return cudaErrorInvalidValue;
     const size_t smem = nr ? (sizeof(V) * (NT / 32)) << nr : 0;
     V* dst = (V*)(g + nr ? partials : out);
-    k_bitsums<V, S, SCALE><<<1u << g, NT, smem, s>>>(st, n, g, nr, dst, scale, err, err_out);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_after(k_bitsums<V, S, SCALE>, 1u << g, NT, smem, s, st, n, g, nr, dst, scale, err, err_out);
     if (e != cudaSuccess || g + nr == 0) return e;
-    k_bitsums_finish<V><<<1 + 2 * n - first, NT, 0, s>>>((const V*)partials, g, first, (V*)out);
-    return cudaGetLastError();
+    return launch_after(k_bitsums_finish<V>, 1 + 2 * n - first, NT, 0, s, (const V*)partials, g, first, (V*)out);
 }
 
 }  // namespace

@@ -10,6 +10,26 @@
 
 namespace kate {
 
+// Launches a kernel that may start before the one before it in the stream has
+// finished, for kernels that call wait_for_previous (k_common.cuh) before
+// they touch any memory that one writes or reads. It hides the launch gap
+// between the dependent kernels of a run (about 1.5 us each).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_after(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                         Args... args) {
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<KArgs>(args)...);
+}
+
 // Product-state initialisation value table: v[b][p] is the factor for
 // physical bit p having value b.
 struct ProductInit {
