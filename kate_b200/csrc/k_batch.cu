@@ -95,23 +95,29 @@ constexpr uint32_t BLK_REGION = 1024 + BLK_IMG + BLK_PROG;
 static_assert(sizeof(BlockProg) % 8 == 0, "BlockProg is copied as 8-byte words");
 // Per CTA, for the whole launch (complex64 batches with block programs):
 // the products' mbarrier and its phase, the TMEM columns, the wait flag.
-__shared__ uint64_t blk_mbar, blk_mbar_img;
-__shared__ uint32_t blk_tmem, blk_phase, blk_phase_img;
+__shared__ uint64_t blk_mbar[2], blk_mbar_img;  // products' mbarrier of each group
+__shared__ uint32_t blk_tmem, blk_phase[2], blk_phase_img;
 __shared__ int blk_abort;
 
 // A complex64 tensor-core block pass over cosets [c0, c1) of one circuit
 // (the BatchProg's BPROG_BLOCK program): the BlockProg and its operand
 // images into shared memory, then per coset the staging tile (loaded, or
 // the tile of |0...0> for a circuit's first pass), the blocks, the
-// write-back. The two batch tile buffers are the double-buffered staging
-// tiles. Loads and stores go through L2 only (other SMs wrote the state
-// earlier in this launch). Returns false when a product wait gave up.
+// write-back. The two batch tile buffers are the staging tiles. Loads and
+// stores go through L2 only (other SMs wrote the state earlier in this
+// launch). Returns false when a product wait gave up.
+// G = 128: two groups of threads take alternate cosets, each with its buffer
+// and TMEM columns, as the simulator's pass kernel does: for tasks of two
+// cosets and more (17 qubits and up; 192 circuits of 10 to 20 qubits take 6.7
+// ms in place of 7.3). G = 256: the whole CTA works on the task's one coset,
+// whose latency is what a small circuit waits for.
+template <int G>
 __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const unsigned char* blob, uint32_t c0,
                                         uint32_t c1, bool first) {
-    const uint32_t t = threadIdx.x;
-    const uint32_t tmem = blk_tmem, mbar = blk::smem_u32(&blk_mbar);
+    const uint32_t t = threadIdx.x, grp = t / G;
+    const uint32_t tmem = blk_tmem + grp * blk::TMEM_COLS, mbar = blk::smem_u32(&blk_mbar[grp]);
     int* abort_flag = &blk_abort;
-    uint32_t phase = blk_phase;  // every thread keeps the same copy; thread 0 stores it back
+    uint32_t phase = blk_phase[grp];  // every thread of the group keeps the same copy; its first one stores it back
     unsigned char* raw = batch_smem_raw + 2 * TS * sizeof(float2);
     const uint32_t rawa = blk::smem_u32(raw);
     const uint32_t bbase = (rawa + 1023u) & ~1023u;
@@ -127,55 +133,36 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     const bool img_ok = blk::load_images(P.nblocks, [&](int b) { return src + P.bimg[b]; }, bbase,
                                          blk::smem_u32(&blk_mbar_img), phase_img);
     if (!img_ok) *abort_flag = 1;
-    blk::Pass<NT> X;
+    blk::Pass<G> X;
     blk::setup(P, X);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    float2* S0 = reinterpret_cast<float2*>(batch_smem_raw);
-    const uint32_t sb0 = blk::smem_u32(batch_smem_raw);
+    float2* S = reinterpret_cast<float2*>(batch_smem_raw) + grp * TS;
+    const uint32_t sb = blk::smem_u32(batch_smem_raw) + grp * blk::S_BYTES;
     bool ok = true;
-    if (first) {
-        for (uint32_t c = c0; c < c1 && ok; c++) {
-            const uint64_t cb = blk::coset_base(P, c);
-            blk::zero_tile<NT>(S0, cb == 0);
-            __syncthreads();
-            ok = blk::apply_blocks(P, X, S0, bbase, tmem, mbar, phase, abort_flag);
-            if (ok) blk::store_tile<true>(P, X, st, cb, S0);
-            __syncthreads();
+    for (uint32_t c = c0 + grp; c < c1; c += NT / G) {
+        const uint64_t cb = blk::coset_base(P, c);
+        if (first) {
+            if (cb) {
+                blk::store_zero<true>(X, st, cb);
+                continue;
+            }
+            blk::zero_tile<G>(S, true);
+        } else {
+            blk::load_tile<true>(st, cb, sb, X);
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
         }
-        if (t == 0) {
-            blk_phase = phase;
-            blk_phase_img = phase_img;
-        }
-        return ok;
+        blk::group_bar<G>();
+        ok = blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag);
+        if (!ok) break;
+        blk::store_tile<true>(P, X, st, cb, S);
+        blk::group_bar<G>();
     }
-    blk::load_tile<true>(st, blk::coset_base(P, c0), sb0, X);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    uint32_t it = 0;
-    for (uint32_t c = c0; c < c1; c++, it++) {
-        const uint32_t cur = it & 1u;
-        float2* S = S0 + cur * TS;
-        // The other buffer was last read by the previous tile's write-back,
-        // closed by the barrier at the end of that iteration.
-        if (c + 1 < c1) blk::load_tile<true>(st, blk::coset_base(P, c + 1), sb0 + (cur ^ 1u) * blk::S_BYTES, X);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        __syncthreads();
-        if (!blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag)) {
-            ok = false;
-            break;
-        }
-        blk::store_tile<true>(P, X, st, blk::coset_base(P, c), S);
-        __syncthreads();
-    }
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();
-    if (t == 0) {
-        blk_phase = phase;
-        blk_phase_img = phase_img;
-    }
-    return ok;
+    if (t % G == 0) blk_phase[grp] = phase;
+    if (t == 0) blk_phase_img = phase_img;
+    // Whether any group's wait gave up: every thread leaves with the same answer.
+    return __syncthreads_and(ok) != 0;
 }
 
 // The register-staged program as a call of its own, so that its registers
@@ -427,14 +414,15 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
     if constexpr (TB) {
         {
             if (t == 0) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar)) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar[0])) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar[1])) : "memory");
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar_img)) : "memory");
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
                 blk_abort = 0;
-                blk_phase = 0;
+                blk_phase[0] = blk_phase[1] = 0;
                 blk_phase_img = 0;
             }
-            blk::tmem_alloc(&blk_tmem, blk::TMEM_COLS);
+            blk::tmem_alloc(&blk_tmem, 2 * blk::TMEM_COLS);
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -472,7 +460,9 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
         if constexpr (TB) block_pass = K.kind == BT_PASS && (progs[K.prog].flags & BPROG_BLOCK);
         if (block_pass) {
             if constexpr (TB) {
-                if (!block_task(arena + circs[K.circ].off, progs[K.prog], blob, K.c0, K.c1, K.first != 0)) {
+                float2* st = arena + circs[K.circ].off;
+                if (!(K.c1 - K.c0 >= 2 ? block_task<128>(st, progs[K.prog], blob, K.c0, K.c1, K.first != 0)
+                                       : block_task<NT>(st, progs[K.prog], blob, K.c0, K.c1, K.first != 0))) {
                     if (t == 0) atomicExch(err, 1);
                     break;
                 }
@@ -542,7 +532,7 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
             atomicAdd(done + K.circ, 1);
         }
     }
-    if constexpr (TB) blk::tmem_free(blk_tmem, blk::TMEM_COLS);
+    if constexpr (TB) blk::tmem_free(blk_tmem, 2 * blk::TMEM_COLS);
 }
 
 template <typename C2, bool TB>

@@ -442,11 +442,16 @@ __device__ __forceinline__ void store_tile(const BlockProg& P, const Pass<G>& X,
 
 // Zeros to every amplitude of a coset (a run from |0...0>: cosets other than
 // the first stay zero under any blocks).
-template <int G>
+template <bool CG, int G>
 __device__ __forceinline__ void store_zero(const Pass<G>& X, float2* st, uint64_t cb) {
     float2* dst = st + cb + X.dT;
+    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int j = 0; j < Pass<G>::NJ; j++) *reinterpret_cast<float4*>(dst + X.dH(j)) = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < Pass<G>::NJ; j++) {
+        float4* p = reinterpret_cast<float4*>(dst + X.dH(j));
+        if (CG) __stcg(p, z);
+        else *p = z;
+    }
 }
 
 }  // namespace blk

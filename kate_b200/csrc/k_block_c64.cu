@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(NT, 2)
         const uint64_t cb = coset_base(P, c);
         if (from_zero) {
             if (cb) {
-                store_zero(X, st, cb);
+                store_zero<false>(X, st, cb);
                 continue;
             }
             zero_tile<G>(S, true);
