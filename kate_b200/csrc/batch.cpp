@@ -390,15 +390,25 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
         std::vector<DevOp>().swap(P.sops);
     });
 
-    // Task queue. Large circuits, window by window, level by level; small
+    // Task queue. Large circuits, window by window, a level at a time; small
     // circuits spread evenly between them (they depend on nothing, so they
     // fill the waits at level boundaries): small circuit s goes right after
     // the first L*s/Sn large tasks, L large tasks in all.
     std::vector<int> large, small;
     for (size_t i = 0; i < np; i++) (packs[i].small ? small : large).push_back((int)i);
-    auto pass_tasks = [&](const CircPack& P) -> uint64_t {
+    // Cosets per pass task: at most `chunk`, and a level split into at most
+    // `split` tasks: 16 when there are few circuits, so that a level spreads
+    // over several CTAs, fewer when the circuits alone keep two waves of CTAs
+    // busy (300 resident CTAs): a task costs about 19 us beside its cosets'
+    // 4.7 us each (dequeuing, descriptors, operand images or tables, the
+    // dependency's round trip).
+    const uint32_t split = (uint32_t)std::min<size_t>(16, std::max<size_t>(1, 600 / std::max<size_t>(1, large.size())));
+    auto pass_cosets = [&](const CircPack& P) -> uint32_t {
         const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS);
-        const uint32_t cch = std::max<uint32_t>(1, std::min<uint32_t>(chunk, ncos / 16));
+        return std::max<uint32_t>(1, std::min<uint32_t>(chunk, ncos / split));
+    };
+    auto pass_tasks = [&](const CircPack& P) -> uint64_t {
+        const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS), cch = pass_cosets(P);
         return (ncos + cch - 1) / cch;
     };
     auto zred_tasks = [&](const CircPack& P) -> uint64_t {
@@ -436,45 +446,63 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
                 w1++;
             } while (w1 < large.size() && (opt.window_bytes == 0 ||
                                            bytes + (1ull << packs[large[w1]].n_sim) * S->amp_bytes() <= opt.window_bytes));
-            size_t maxlev = 0;
-            for (size_t k = w0; k < w1; k++) maxlev = std::max(maxlev, packs[large[k]].progs.size() + 1);
-            for (size_t lev = 0; lev < maxlev; lev++)
-                for (size_t k = w0; k < w1; k++) {
-                    const int ci = large[k];
-                    const CircPack& P = packs[ci];
-                    const size_t nprog = P.progs.size();
-                    if (lev > nprog) continue;
-                    const int before = need[k];
-                    if (lev < nprog) {
-                        const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS);
-                        // Small states: fewer cosets per task, so a level spreads over several CTAs.
-                        const uint32_t cch = std::max<uint32_t>(1, std::min<uint32_t>(chunk, ncos / 16));
-                        for (uint32_t c0 = 0; c0 < ncos; c0 += cch) {
-                            BatchTask t{};
-                            t.kind = BT_PASS;
-                            t.circ = ci;
-                            t.prog = prog0[ci] + (int)lev;
-                            t.c0 = c0;
-                            t.c1 = std::min<uint32_t>(ncos, c0 + cch);
-                            t.need = before;
-                            t.first = lev == 0;
-                            push_large(t);
-                            need[k]++;
-                        }
-                    } else {
-                        const uint32_t nch = (uint32_t)std::max<uint64_t>(1, (1ull << P.n_sim) >> 16);
-                        for (uint32_t c0 = 0; c0 < nch; c0 += zchunks) {
-                            BatchTask t{};
-                            t.kind = BT_ZRED;
-                            t.circ = ci;
-                            t.c0 = c0;
-                            t.c1 = std::min<uint32_t>(nch, c0 + zchunks);
-                            t.need = before;
-                            push_large(t);
-                            need[k]++;
-                        }
+            // The window's levels in the order of the share of their circuit
+            // that they complete, so that circuits of few and of many levels
+            // end together: level by level instead, the widest circuits were
+            // left to run their last levels alone, with too few tasks for the
+            // CTAs and a wait at every one. A circuit's next level then comes
+            // (all tasks) / (its levels) tasks later, which is what its
+            // dependency waits have to be covered by. Larger states first
+            // among equals.
+            struct Level {
+                uint64_t at;  // share completed before it ends, in 2^-32
+                int n;
+                uint32_t k, lev;
+            };
+            std::vector<Level> order;
+            for (size_t k = w0; k < w1; k++) {
+                const uint64_t nlev = packs[large[k]].progs.size() + 1;
+                for (uint64_t lev = 0; lev < nlev; lev++)
+                    order.push_back({((2 * lev + 1) << 32) / (2 * nlev), packs[large[k]].n_sim, (uint32_t)k, (uint32_t)lev});
+            }
+            std::sort(order.begin(), order.end(), [](const Level& a, const Level& b) {
+                return a.at != b.at ? a.at < b.at : a.n != b.n ? a.n > b.n : a.k < b.k;
+            });
+            for (const Level& o : order) {
+                const size_t k = o.k, lev = o.lev;
+                const int ci = large[k];
+                const CircPack& P = packs[ci];
+                const size_t nprog = P.progs.size();
+                const int before = need[k];
+                if (lev < nprog) {
+                    const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS);
+                    const uint32_t cch = pass_cosets(P);
+                    for (uint32_t c0 = 0; c0 < ncos; c0 += cch) {
+                        BatchTask t{};
+                        t.kind = BT_PASS;
+                        t.circ = ci;
+                        t.prog = prog0[ci] + (int)lev;
+                        t.c0 = c0;
+                        t.c1 = std::min<uint32_t>(ncos, c0 + cch);
+                        t.need = before;
+                        t.first = lev == 0;
+                        push_large(t);
+                        need[k]++;
+                    }
+                } else {
+                    const uint32_t nch = (uint32_t)std::max<uint64_t>(1, (1ull << P.n_sim) >> 16);
+                    for (uint32_t c0 = 0; c0 < nch; c0 += zchunks) {
+                        BatchTask t{};
+                        t.kind = BT_ZRED;
+                        t.circ = ci;
+                        t.c0 = c0;
+                        t.c1 = std::min<uint32_t>(nch, c0 + zchunks);
+                        t.need = before;
+                        push_large(t);
+                        need[k]++;
                     }
                 }
+            }
             w0 = w1;
         }
         while (si < Sn) push_small();  // only when there are no large circuits
