@@ -308,15 +308,28 @@ __device__ __noinline__ void chunk_prefix(double* psum, uint32_t nch, double* re
     if (t == 0) psum[2 * nch] = total;
 }
 
+// Sum of v over the warp's lanes, the same on every lane (a fixed tree).
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // Inverse-CDF sampling over chunks [ch0, ch1): shot s (uniforms u ascending)
 // targets x = u * total; it falls in chunk ch when pre[ch] <= x < pre[ch] +
 // sum[ch] (targets at or past the total go to the last chunk). Inside a
-// chunk, thread t owns a contiguous run of amplitudes; a block scan of the
-// runs' sums locates each target's run, whose owner walks it.
+// chunk, the sums of its runs of 256 amplitudes (a warp each) and their
+// prefix come first; then every warp takes shots of its own: the prefix names
+// the run, whose 256 amplitudes the warp reads at once and walks 32 at a
+// time. With a thread owning 256 amplitudes and walking them one load after
+// another, 1024 shots of a 16-qubit state took milliseconds, most of a served
+// request's time. The tile buffers hold the prefix.
 template <typename C2>
 __device__ __noinline__ void sample_chunks(const C2* st, int n, uint32_t ch0, uint32_t ch1, const double* psum,
                                            const double* unif, int shots, uint64_t* out, double* red, int* srange) {
-    const uint32_t t = threadIdx.x;
+    constexpr uint32_t RUN = 256, FULL = 0xffffffffu;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    double* pre = reinterpret_cast<double*>(batch_smem_raw);
     const uint64_t dim = 1ull << n;
     const uint32_t nch = (uint32_t)(dim >> 16 ? dim >> 16 : 1);
     const double total = psum[2 * nch];
@@ -346,33 +359,71 @@ __device__ __noinline__ void sample_chunks(const C2* st, int n, uint32_t ch0, ui
         __syncthreads();
         if (s0 >= s1) continue;
         const uint64_t x0 = (uint64_t)ch << 16;
-        const uint64_t len = dim - x0 < (1ull << 16) ? dim - x0 : (1ull << 16);
-        const uint64_t per = (len + NT - 1) / NT;
-        const uint64_t a0 = x0 + (t * per < len ? t * per : len), a1 = x0 + ((t + 1) * per < len ? (t + 1) * per : len);
-        double w = 0.0;
-        for (uint64_t x = a0; x < a1; x++) {
-            const double2 a = ldst(st + x);
-            w += a.x * a.x + a.y * a.y;
-        }
-        double btot;
-        const double base = block_exscan(w, red, &btot);
-        const bool tail = (t == NT - 1) || (a1 == x0 + len);
-        for (int s = s0; s < s1; s++) {
-            const double y = unif[s] * total - lo_v;
-            const bool mine = (y >= base && y < base + w) || (tail && y >= base + w && a1 > a0 && a1 == x0 + len);
-            if (!mine || a1 <= a0) continue;
-            double acc = base;
-            uint64_t pick = a1 - 1;
-            for (uint64_t x = a0; x < a1; x++) {
-                const double2 a = ldst(st + x);
-                const double p = a.x * a.x + a.y * a.y;
-                acc += p;
-                if (acc > y && p > 0.0) {
-                    pick = x;
-                    break;
-                }
+        const uint32_t len = (uint32_t)(dim - x0 < (1ull << 16) ? dim - x0 : (1ull << 16));
+        const uint32_t nrun = len / RUN;  // states of 12 qubits and more: 16 to 256
+        const C2* p = st + x0;
+        auto probs = [&](uint32_t run, double (&v)[8]) {
+#pragma unroll
+            for (uint32_t k = 0; k < 8; k++) {
+                const double2 a = ldst(p + run * RUN + 32 * k + lane);
+                v[k] = a.x * a.x + a.y * a.y;
             }
-            out[s] = pick;
+        };
+        for (uint32_t r = warp; r < nrun; r += NT / 32) {
+            double v[8];
+            probs(r, v);
+            const double w = warp_sum(((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+            if (lane == 0) pre[r] = w;
+        }
+        __syncthreads();
+        double tot;
+        const double base = block_exscan(t < nrun ? pre[t] : 0.0, red, &tot);
+        if (t < nrun) pre[t] = base;
+        __syncthreads();
+        for (int s = s0 + (int)warp; s < s1; s += NT / 32) {
+            const double y = unif[s] * total - lo_v;
+            // Last run whose prefix is at most y: eight runs per lane, then
+            // the runs of that lane.
+            const uint32_t hi8 = __ballot_sync(FULL, 8 * lane < nrun && pre[8 * lane] <= y);
+            const uint32_t g = hi8 ? 8u * (31u - (uint32_t)__clz((int)hi8)) : 0u;
+            const uint32_t lo8 = __ballot_sync(FULL, lane < 8 && g + lane < nrun && pre[g + lane] <= y);
+            uint32_t r = g + (lo8 ? 31u - (uint32_t)__clz((int)lo8) : 0u);
+            uint32_t pick = 0;
+            for (bool found = false; !found;) {
+                double v[8], acc = pre[r];
+                uint32_t lastnz = 0;
+                bool any = false;
+                probs(r, v);
+                double w[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) w[k] = warp_sum(v[k]);
+#pragma unroll
+                for (uint32_t k = 0; k < 8; k++) {
+                    if (found) continue;
+                    const uint32_t nz = __ballot_sync(FULL, v[k] > 0.0);
+                    if (acc + w[k] > y && nz) {
+                        double inc = v[k];
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const double u = __shfl_up_sync(FULL, inc, o);
+                            if (lane >= (uint32_t)o) inc += u;
+                        }
+                        // The tree's sum may pass y by a rounding that the
+                        // scan does not: then the last nonzero amplitude.
+                        const uint32_t hit = __ballot_sync(FULL, v[k] > 0.0 && acc + inc > y);
+                        pick = r * RUN + 32 * k + (hit ? (uint32_t)__ffs((int)hit) - 1u : 31u - (uint32_t)__clz((int)nz));
+                        found = true;
+                    }
+                    if (nz) lastnz = r * RUN + 32 * k + 31u - (uint32_t)__clz((int)nz), any = true;
+                    acc += w[k];
+                }
+                // y at or past the run's end (rounding between the sums): the
+                // last amplitude of nonzero probability at or before it.
+                if (!found && any) pick = lastnz;
+                if (found || any || r == 0) break;
+                r--;
+            }
+            if (lane == 0) out[s] = x0 + pick;
         }
         __syncthreads();
     }

@@ -332,12 +332,18 @@ struct ServerImpl {
         resident -= (1ull << r->pack.n_sim) * amp_bytes();
     }
 
+    // Cosets per pass task of r: small states one, so that a level spreads
+    // over several CTAs.
+    uint32_t pass_cosets(const Req* r) const {
+        return std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)std::max(1, opt.chunk), r->ncos / 64));
+    }
+
     // Estimated latency of level a of r in microseconds (the levels of a
     // request run one after another inside a step): waves of tasks over the
     // CTAs, about 20 us per 4096-amplitude tile pass plus 5 us per task.
     double level_latency_us(const Req* r, int a) const {
         if (a < r->npass) {
-            const uint32_t ch = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)std::max(1, opt.chunk), r->ncos / 64));
+            const uint32_t ch = pass_cosets(r);
             const uint64_t tasks = (r->ncos + ch - 1) / ch;
             const uint64_t waves = (tasks + grid - 1) / std::max(1, grid);
             return (double)waves * (20.0 * ch + 5.0);
@@ -426,56 +432,67 @@ struct ServerImpl {
             if (L > 0) sched.push_back({r, L});
         }
         if (sched.empty()) return "";
-        // Task list: requests grouped by tiles per pass (small groups first),
-        // level-major inside a group.
-        std::stable_sort(sched.begin(), sched.end(),
-                         [](const auto& a, const auto& b) { return a.first->ncos < b.first->ncos; });
+        // Task list: every scheduled level of every request in the order of
+        // the time its turn is expected, the latencies of the request's
+        // levels before it added up. A CTA that takes a task early holds it
+        // while it waits for the level before, so tasks should come up about
+        // when they can run: queued request group by request group instead,
+        // all CTAs held the later levels of the small requests while the
+        // large ones, queued behind them, had not begun (48 requests of 12 to
+        // 21 qubits: four steps of 3 to 4.4 ms).
         std::vector<BatchCirc> circs;
         std::vector<BatchTask> tasks;
         std::vector<int> cnt(sched.size(), 0);
-        for (size_t i = 0; i < sched.size(); i++) circs.push_back(sched[i].first->circ);
-        size_t g0 = 0;
-        const int chunk = std::max(1, opt.chunk), zch = std::max(1, opt.zchunks), sch = std::max(1, opt.schunks);
-        while (g0 < sched.size()) {
-            size_t g1 = g0;
-            int maxL = 0;
-            while (g1 < sched.size() && sched[g1].first->ncos == sched[g0].first->ncos) {
-                maxL = std::max(maxL, sched[g1].second);
-                g1++;
+        struct Turn {
+            double at;
+            int i, l;
+        };
+        std::vector<Turn> turns;
+        for (size_t i = 0; i < sched.size(); i++) {
+            Req* r = sched[i].first;
+            circs.push_back(r->circ);
+            double at = 0.0;
+            for (int l = 0; l < sched[i].second; l++) {
+                turns.push_back({at, (int)i, l});
+                at += level_latency_us(r, r->next_level + l);
             }
-            for (int l = 0; l < maxL; l++)
-                for (size_t i = g0; i < g1; i++) {
-                    Req* r = sched[i].first;
-                    if (l >= sched[i].second) continue;
-                    const int a = r->next_level + l;
-                    const int before = cnt[i];
-                    auto add = [&](int kind, uint32_t c0, uint32_t c1) {
-                        BatchTask t{};
-                        t.kind = kind;
-                        t.circ = (int32_t)i;
-                        t.c0 = c0;
-                        t.c1 = c1;
-                        t.need = before;
-                        if (kind == BT_PASS) {
-                            t.prog = (int32_t)(r->prog0 + a);
-                            t.first = a == 0;
-                        }
-                        tasks.push_back(t);
-                        cnt[i]++;
-                    };
-                    if (a < r->npass) {
-                        // Small states: one coset per task, so a level spreads over several CTAs.
-                        const uint32_t ch = std::max<uint32_t>(1, std::min<uint32_t>(chunk, r->ncos / 64));
-                        for (uint32_t c0 = 0; c0 < r->ncos; c0 += ch) add(BT_PASS, c0, std::min(r->ncos, c0 + ch));
-                    } else if (a == r->npass) {
-                        for (uint32_t c0 = 0; c0 < r->nch; c0 += zch) add(BT_ZRED, c0, std::min(r->nch, c0 + zch));
-                    } else if (a == r->npass + 1) {
-                        add(BT_PREFIX, 0, 1);
-                    } else {
-                        for (uint32_t c0 = 0; c0 < r->nch; c0 += sch) add(BT_SAMPLE, c0, std::min(r->nch, c0 + sch));
-                    }
+        }
+        // At the same time the request with the longer way to go first.
+        std::vector<double> end(sched.size(), 0.0);
+        for (const Turn& t : turns) end[t.i] = std::max(end[t.i], t.at);
+        std::sort(turns.begin(), turns.end(), [&](const Turn& a, const Turn& b) {
+            return a.at != b.at ? a.at < b.at : end[a.i] != end[b.i] ? end[a.i] > end[b.i] : a.i != b.i ? a.i < b.i : a.l < b.l;
+        });
+        const int zch = std::max(1, opt.zchunks), sch = std::max(1, opt.schunks);
+        for (const Turn& turn : turns) {
+            const int i = turn.i;
+            Req* r = sched[i].first;
+            const int a = r->next_level + turn.l;
+            const int before = cnt[i];
+            auto add = [&](int kind, uint32_t c0, uint32_t c1) {
+                BatchTask t{};
+                t.kind = kind;
+                t.circ = (int32_t)i;
+                t.c0 = c0;
+                t.c1 = c1;
+                t.need = before;
+                if (kind == BT_PASS) {
+                    t.prog = (int32_t)(r->prog0 + a);
+                    t.first = a == 0;
                 }
-            g0 = g1;
+                tasks.push_back(t);
+                cnt[i]++;
+            };
+            if (a < r->npass) {
+                const uint32_t ch = pass_cosets(r);
+                for (uint32_t c0 = 0; c0 < r->ncos; c0 += ch) add(BT_PASS, c0, std::min(r->ncos, c0 + ch));
+            } else if (a == r->npass) {
+                for (uint32_t c0 = 0; c0 < r->nch; c0 += zch) add(BT_ZRED, c0, std::min(r->nch, c0 + zch));
+            } else if (a == r->npass + 1) {
+                add(BT_PREFIX, 0, 1);
+            } else {
+                for (uint32_t c0 = 0; c0 < r->nch; c0 += sch) add(BT_SAMPLE, c0, std::min(r->nch, c0 + sch));
+            }
         }
         if (tasks.size() > (size_t)INT32_MAX) return "step has too many tasks";
         std::string e = ensure((void**)&S.d_tasks, &S.tasks_cap, tasks.size() * sizeof(BatchTask));
