@@ -17,9 +17,9 @@
 //   BT_PREFIX exclusive prefix of a circuit's chunk sums;
 //   BT_SAMPLE inverse-CDF sampling of the shots falling in a chunk range.
 // Finished tasks bump their circuit's counter after a memory fence. Tasks
-// are queued level by level per circuit, so a task waits only on tasks
-// dequeued before it: every CTA that holds a task can finish it, whatever
-// the number of resident CTAs.
+// are queued in level order per circuit, so a task waits only on tasks
+// dequeued before it: every CTA can finish the task it runs, whatever the
+// number of resident CTAs.
 // C2 is the amplitude type: float2 (complex64, FP32 arithmetic) or double2
 // (complex128, FP64 arithmetic). <Z> sums are FP64.
 #include <cuda_runtime.h>
@@ -99,22 +99,81 @@ __shared__ uint64_t blk_mbar[2], blk_mbar_img;  // products' mbarrier of each gr
 __shared__ uint32_t blk_tmem, blk_phase[2], blk_phase_img;
 __shared__ int blk_abort;
 
+// Waits (time-bounded) until `need` tasks of the circuit have finished; every
+// thread returns the same answer, after a barrier. *abort (shared) is set
+// when the wait gave up.
+__device__ __forceinline__ bool wait_dep(const int* done, int need, int* err, unsigned long long wait_ns, int* abort) {
+    if (threadIdx.x == 0 && need > 0) {
+        const unsigned long long t0 = now_ns();
+        while (*((volatile const int*)done) < need) {
+            if (now_ns() - t0 > wait_ns || *((volatile int*)err)) {
+                *abort = 1;
+                atomicExch(err, 1);
+                break;
+            }
+            __nanosleep(256);
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return *abort == 0;
+}
+
+// The task queue as a CTA sees it. A CTA takes its next task in the last step
+// of the current one, by one thread and in two parts: the index (an atomic)
+// and, once that is there, the descriptor's copy into shared memory, so that
+// neither round trip is on the CTA's path (192 complex64 circuits of 10 to 20
+// qubits: 5.5 ms; 6.1 ms with both between two tasks and the dependency waited
+// for before a task's tables and operand images were in place). Not earlier: a
+// task taken while the current one still waits or runs for long is kept from
+// the other CTAs (5.6 ms when it was taken at the current one's start, and 48
+// requests to the server took 11.6 ms in place of 8.7).
+// Of the unfinished tasks the one taken first is always some CTA's current
+// one (a CTA runs its tasks in the order it took them) and waits only on
+// tasks taken before it: nothing can wait in a circle.
+__shared__ __align__(16) BatchTask q_task[2];  // this task and the next
+__shared__ int q_idx[2];
+__shared__ const BatchTask* q_tasks;
+__shared__ int *q_head, *q_err;
+__shared__ int q_n;
+constexpr uint32_t TAKER = NT - 32;  // the thread that takes the next task
+static_assert(sizeof(BatchTask) == 32, "a descriptor is two 16-byte copies");
+
+__device__ __forceinline__ int take_index() {
+    // After a failed wait anywhere, every CTA stops at its next task.
+    return *((volatile int*)q_err) ? q_n : atomicAdd(q_head, 1);
+}
+__device__ __forceinline__ void fetch_task(int i, uint32_t slot) {
+    q_idx[slot] = i;
+    if (i < q_n) {
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(&q_task[slot]);
+        const char* src = reinterpret_cast<const char*>(q_tasks + i);
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d + 16u), "l"(src + 16) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+
 // A complex64 tensor-core block pass over cosets [c0, c1) of one circuit
 // (the BatchProg's BPROG_BLOCK program): the BlockProg and its operand
 // images into shared memory, then per coset the staging tile (loaded, or
 // the tile of |0...0> for a circuit's first pass), the blocks, the
 // write-back. The two batch tile buffers are the staging tiles. Loads and
 // stores go through L2 only (other SMs wrote the state earlier in this
-// launch). Returns false when a product wait gave up.
+// launch). The dependency is waited for once everything that does not depend
+// on it is in place. Returns false when a wait gave up.
 // G = 128: two groups of threads take alternate cosets, each with its buffer
 // and TMEM columns, as the simulator's pass kernel does: for tasks of two
 // cosets and more (17 qubits and up; 192 circuits of 10 to 20 qubits take 6.7
 // ms in place of 7.3). G = 256: the whole CTA works on the task's one coset,
 // whose latency is what a small circuit waits for.
 template <int G>
-__device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const unsigned char* blob, uint32_t c0,
-                                        uint32_t c1, bool first) {
+__device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const unsigned char* blob, uint32_t slot,
+                                        const int* done, unsigned long long wait_ns, int* abort) {
+    const BatchTask& K = q_task[slot];
     const uint32_t t = threadIdx.x, grp = t / G;
+    const uint32_t c0 = K.c0, c1 = K.c1;
+    const bool first = K.first != 0;
     const uint32_t tmem = blk_tmem + grp * blk::TMEM_COLS, mbar = blk::smem_u32(&blk_mbar[grp]);
     int* abort_flag = &blk_abort;
     uint32_t phase = blk_phase[grp];  // every thread of the group keeps the same copy; its first one stores it back
@@ -136,15 +195,22 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     blk::Pass<G> X;
     blk::setup(P, X);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
+    if (!wait_dep(done, K.need, q_err, wait_ns, abort)) {
+        if (t == 0) blk_phase_img = phase_img;
+        return false;
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     float2* S = reinterpret_cast<float2*>(batch_smem_raw) + grp * TS;
     const uint32_t sb = blk::smem_u32(batch_smem_raw) + grp * blk::S_BYTES;
     bool ok = true;
     for (uint32_t c = c0 + grp; c < c1; c += NT / G) {
         const uint64_t cb = blk::coset_base(P, c);
+        const bool take = t == TAKER && c + NT / G >= c1;  // the last group's last coset
+        int next = 0;
+        if (take) next = take_index();
         if (first) {
             if (cb) {
+                if (take) fetch_task(next, slot ^ 1u);
                 blk::store_zero<true>(X, st, cb);
                 continue;
             }
@@ -153,6 +219,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
             blk::load_tile<true>(st, cb, sb, X);
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
         }
+        if (take) fetch_task(next, slot ^ 1u);
         blk::group_bar<G>();
         ok = blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag);
         if (!ok) break;
@@ -453,7 +520,6 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
     // other one), then the program tables.
     C2* tile = reinterpret_cast<C2*>(batch_smem_raw);
     TileTables<C2>& T = *reinterpret_cast<TileTables<C2>*>(batch_smem_raw + 2 * TS * sizeof(C2));
-    __shared__ int s_task;
     __shared__ int s_abort;
     __shared__ uint8_t s_zbit[40];
     __shared__ int s_range[2];
@@ -479,41 +545,34 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
     }
-    for (;;) {
-        if (t == 0) {
-            // After a failed wait anywhere, every CTA stops at its next task.
-            s_task = *((volatile int*)err) ? ntasks : atomicAdd(head, 1);
-            s_abort = 0;
-        }
-        __syncthreads();
-        const int ti = s_task;
-        if (ti >= ntasks) break;
-        const BatchTask K = tasks[ti];
-        if (t == 0 && K.need > 0) {
-            const unsigned long long t0 = now_ns();
-            while (*((volatile int*)(done + K.circ)) < K.need) {
-                if (now_ns() - t0 > wait_ns || *((volatile int*)err)) {
-                    s_abort = 1;
-                    atomicExch(err, 1);
-                    break;
-                }
-                __nanosleep(256);
-            }
-            __threadfence();
-        }
-        if (t < 40) s_zbit[t] = circs[K.circ].zbit[t];
-        __syncthreads();
-        if (s_abort) break;
-        const int nz = circs[K.circ].n;
-        const int64_t zoff = circs[K.circ].zoff;
-
+    if (t == TAKER) {
+        s_abort = 0;
+        q_tasks = tasks;
+        q_head = head;
+        q_err = err;
+        q_n = ntasks;
+        fetch_task(take_index(), 0);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    for (uint32_t now = 0;; now ^= 1u) {
+        if (q_idx[now] >= q_n) break;
+        const BatchTask& K = q_task[now];
+        if (t == TAKER) q_idx[now ^ 1u] = -1;  // not taken yet
+        auto ready = [&] { return wait_dep(done + K.circ, K.need, err, wait_ns, &s_abort); };
+        const bool pass = K.kind == BT_PASS;
         bool block_pass = false;
-        if constexpr (TB) block_pass = K.kind == BT_PASS && (progs[K.prog].flags & BPROG_BLOCK);
+        if constexpr (TB) block_pass = pass && (progs[K.prog].flags & BPROG_BLOCK);
+        if (!pass) {
+            if (t < 40) s_zbit[t] = circs[K.circ].zbit[t];
+            if (!ready()) break;
+        }
         if (block_pass) {
             if constexpr (TB) {
                 float2* st = arena + circs[K.circ].off;
-                if (!(K.c1 - K.c0 >= 2 ? block_task<128>(st, progs[K.prog], blob, K.c0, K.c1, K.first != 0)
-                                       : block_task<NT>(st, progs[K.prog], blob, K.c0, K.c1, K.first != 0))) {
+                const int* dn = done + K.circ;
+                if (!(K.c1 - K.c0 >= 2 ? block_task<128>(st, progs[K.prog], blob, now, dn, wait_ns, &s_abort)
+                                       : block_task<NT>(st, progs[K.prog], blob, now, dn, wait_ns, &s_abort))) {
                     if (t == 0) atomicExch(err, 1);
                     break;
                 }
@@ -531,11 +590,10 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
                 setup_program(T, v, t);
                 setup_io(T, v, t);
             }
+            // The tables are in place: now the dependency.
+            if (pass && !ready()) break;
             const bool pre = !small && !K.first;  // pass task that loads: double-buffered
-            if (pre) {
-                __syncthreads();
-                load_async(T, st, K.c0, tb, t);
-            }
+            if (pre) load_async(T, st, K.c0, tb, t);
             for (int s = 0; s < nsteps; s++) {
                 const BatchProg& P = progs[small ? K.prog + s : K.prog];
                 const uint32_t c = K.c0 + (uint32_t)s;
@@ -557,6 +615,7 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
                         asm volatile("cp.async.wait_group 0;\n" ::: "memory");
                     }
                 }
+                if (t == TAKER && s + 1 == nsteps) fetch_task(take_index(), now ^ 1u);
                 __syncthreads();
                 run_any(T, P, blob, tbc, tilec, cbase, sops, pool, t);
                 if (!small) {
@@ -565,24 +624,31 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
                 }
             }
             __syncthreads();
-            if (small) small_z(tile, nz, s_zbit, red, zout + zoff);
+            if (small) small_z(tile, circs[K.circ].n, s_zbit, red, zout + circs[K.circ].zoff);
         } else {
             const BatchCirc& C = circs[K.circ];
+            const int nz = C.n;
             const uint32_t nch = (uint32_t)(((1ull << nz) >> 16) ? ((1ull << nz) >> 16) : 1);
             if (K.kind == BT_ZRED)
-                zred(arena + C.off, nz, K.c0, K.c1, s_zbit, red, zout + zoff, C.poff >= 0 ? psum + C.poff : nullptr);
+                zred(arena + C.off, nz, K.c0, K.c1, s_zbit, red, zout + C.zoff, C.poff >= 0 ? psum + C.poff : nullptr);
             else if (K.kind == BT_PREFIX)
                 chunk_prefix(psum + C.poff, nch, red);
             else if (K.kind == BT_SAMPLE)
                 sample_chunks(arena + C.off, nz, K.c0, K.c1, psum + C.poff, unif + C.uoff, C.shots, sout + C.soff,
                               red, s_range);
         }
+        if (t == TAKER) {
+            if (q_idx[now ^ 1u] < 0) fetch_task(take_index(), now ^ 1u);  // a task without steps
+            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        }
+        int* const finished = done + K.circ;  // read before the barrier: K's place is the task's after the next
         __syncthreads();
         if (t == 0) {
             __threadfence();
-            atomicAdd(done + K.circ, 1);
+            atomicAdd(finished, 1);
         }
     }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     if constexpr (TB) blk::tmem_free(blk_tmem, 2 * blk::TMEM_COLS);
 }
 
