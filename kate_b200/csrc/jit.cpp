@@ -376,7 +376,6 @@ std::string jit_pass_source(const PassProg& P, const DevOp* sops, std::string* w
         }
     }
     if (first < 0 && !smem_first) return no("no stage");
-    if (smem_first && form != 0) return no("a first pass that starts with a shared-memory op");
     for (int s = 0; s < P.nstages; s++)
         if (!stage_linear(P, s)) return no("stage table not linear");
     Gen g(P);
@@ -621,7 +620,27 @@ std::string jit_pass_source(const PassProg& P, const DevOp* sops, std::string* w
         }
         case SOP_SMEM:
             if (!started) {
-                copy_in();
+                // The start forms put the tile where the copy-in would have
+                // (23 qubits, a first pass that begins with a dense gate:
+                // writing |0...0> and computing every coset of it took 25 +
+                // 199 us, coset 0 alone and zeros elsewhere take 65).
+                if (from_zero) {
+                    // Element 0 sits at offset 0: the swizzle is linear.
+                    for (int j = 0; j < 16; j++)
+                        o << "    sts(tb + ((t | " << hex32((uint32_t)j << 8) << ") << 4), mk("
+                          << (j ? "0.0" : "t == 0 ? 1.0 : 0.0") << ", 0.0));\n";
+                    o << "    __syncthreads();\n";
+                } else if (from_prod) {
+                    // With the coset's factor, which a pass without a later
+                    // stage would not get to.
+                    for (int j = 0; j < 16; j++)
+                        o << "    { const u32 e = t | " << hex32((uint32_t)j << 8) << "; sts(tb + (csw ^ "
+                          << hex32(swz((uint32_t)j << 8) << 4) << "), cmul(qc, cmul(ptl[e & 63u], pth[e >> 6]))); }\n";
+                    o << "    __syncthreads();\n";
+                    g.qc = false;
+                } else {
+                    copy_in();
+                }
                 started = true;
             } else if (open) {
                 store_regs();

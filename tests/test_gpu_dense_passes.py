@@ -68,3 +68,18 @@ def test_compiled_circuits_match_the_interpreter(family):
         sim.execute()
         states.append(sim.state())
     assert np.abs(states[0] - states[1]).max() <= 1e-12
+
+
+@pytest.mark.parametrize("n", [12, 13, 16])
+@pytest.mark.parametrize("sizes,between", [([3], 0), ([4], 1), ([5], 2), ([4, 3, 5], 0), ([5, 4], 4)])
+def test_first_pass_starting_with_a_dense_gate(n, sizes, between, oracle):
+    # It makes |0...0> or the product state itself: no launch besides the passes.
+    g = dense(n, sizes, 31 * n + len(sizes), between)
+    rng = np.random.default_rng(n)
+    tp = np.stack([rng.uniform(0, 1, n), rng.uniform(-np.pi, np.pi, n)], axis=1)
+    sim = K.Simulator(K.Circuit(n, g))
+    assert sim.launches_per_run() == len(sim.pass_kernels())
+    sim.execute()
+    assert np.abs(sim.state() - oracle.simulate(n, g)).max() <= 1e-12
+    sim.execute(K.proba_state(tp))
+    assert np.abs(sim.state() - oracle.simulate(n, g, proba_in=tp)).max() <= 1e-12
