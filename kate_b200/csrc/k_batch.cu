@@ -203,6 +203,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     float2* S = reinterpret_cast<float2*>(batch_smem_raw) + grp * TS;
     const uint32_t sb = blk::smem_u32(batch_smem_raw) + grp * blk::S_BYTES;
     bool ok = true;
+    double unused = 0.0;
     for (uint32_t c = c0 + grp; c < c1; c += NT / G) {
         const uint64_t cb = blk::coset_base(P, c);
         const bool take = t == TAKER && c + NT / G >= c1;  // the last group's last coset
@@ -223,7 +224,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
         blk::group_bar<G>();
         ok = blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag);
         if (!ok) break;
-        blk::store_tile<true>(P, X, st, cb, S);
+        blk::store_tile<true, false>(P, X, st, cb, S, unused);
         blk::group_bar<G>();
     }
     if (t % G == 0) blk_phase[grp] = phase;

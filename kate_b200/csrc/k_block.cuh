@@ -416,12 +416,15 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& 
 
 // Writes the staging tile back with the remap permutation, an amplitude pair
 // per store. st_cg: stores that bypass L1 (the state is read by other SMs
-// later in the same launch).
-template <bool CG, int G>
+// later in the same launch). NORM: adds |a|^2 of this thread's amplitudes to
+// `norm`.
+template <bool CG, bool NORM, int G>
 __device__ __forceinline__ void store_tile(const BlockProg& P, const Pass<G>& X, float2* st, uint64_t cb,
-                                           const float2* S) {
+                                           const float2* S, double& norm) {
     float2* dst = st + cb + X.dT;
     auto put = [&](float2* p, float4 v) {
+        if (NORM)
+            norm += ((double)v.x * v.x + (double)v.y * v.y) + ((double)v.z * v.z + (double)v.w * v.w);
         if (CG) __stcg(reinterpret_cast<float4*>(p), v);
         else *reinterpret_cast<float4*>(p) = v;
     };

@@ -21,6 +21,7 @@
 // per round bit in registers the amplitude form held 128 registers and read
 // 1 GiB in 416 us (2.6 TB/s).
 #include "k_common.cuh"
+#include "k_norm.cuh"
 #include "launch.hpp"
 
 namespace kate {
@@ -234,17 +235,9 @@ __global__ void k_probs(const S* __restrict__ st, uint64_t dim, double* __restri
 
 // ---- renormalisation of complex64 states ----
 // ||psi||^2 in FP64: each CTA sums |a|^2 over a grid-stride range (16-byte
-// loads, two amplitudes each, in a fixed per-thread order), reduces it in a
-// fixed tree, writes its partial; the last CTA to finish adds the partials
-// in a fixed order (deterministic) and writes out[0] = ||psi||^2 and out[1] =
-// 1 / ||psi||, then resets the counter for the next run.
-constexpr int RN_GRID = 148 * 4;
-
-__global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st, uint64_t npairs,
-                                                   double* __restrict__ part, unsigned* __restrict__ count,
-                                                   double* __restrict__ out) {
-    __shared__ double red[256];
-    __shared__ bool last;
+// loads, two amplitudes each, in a fixed per-thread order); finish_norm does
+// the rest.
+__global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st, uint64_t npairs, NormScratch N) {
     let_next_start();
     wait_for_previous();
     const uint32_t t = threadIdx.x;
@@ -263,36 +256,7 @@ __global__ void __launch_bounds__(256) k_norm2_c64(const float4* __restrict__ st
         const float4 v = __ldcs(st + i);
         acc += ((double)v.x * v.x + (double)v.y * v.y) + ((double)v.z * v.z + (double)v.w * v.w);
     }
-    red[t] = acc;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (t < (uint32_t)w) red[t] += red[t + w];
-        __syncthreads();
-    }
-    if (t == 0) {
-        part[blockIdx.x] = red[0];
-        __threadfence();
-        last = atomicAdd(count, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    // Partials by the whole CTA, in a fixed order (one thread adding 592 of
-    // them one after another took 20 us, most of the kernel at 21 qubits).
-    __threadfence();
-    double tot = 0.0;
-    for (uint32_t c = t; c < gridDim.x; c += 256) tot += __ldcg(part + c);
-    red[t] = tot;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (t < (uint32_t)w) red[t] += red[t + w];
-        __syncthreads();
-    }
-    if (t == 0) {
-        tot = red[0];
-        out[0] = tot;
-        out[1] = tot > 0.0 ? 1.0 / sqrt(tot) : 1.0;
-        *count = 0;
-    }
+    finish_norm<256>(acc, N);
 }
 
 // Multiplies every amplitude by the scale the norm kernel wrote (read on
@@ -323,15 +287,12 @@ size_t renorm_scratch_bytes() { return (RN_GRID + 4) * sizeof(double); }
 cudaError_t launch_norm_c64(const void* st, int n, void* scratch, cudaStream_t s) {
     if (n < 1) return cudaErrorInvalidValue;
     const uint64_t npairs = (1ull << n) / 2;
-    double* part = (double*)scratch;
-    double* out = part + RN_GRID;
-    unsigned* count = (unsigned*)(out + 2);
     const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
-    return launch_after(k_norm2_c64, grid, 256, 0, s, (const float4*)st, npairs, part, count, out);
+    return launch_after(k_norm2_c64, grid, 256, 0, s, (const float4*)st, npairs, norm_scratch(scratch));
 }
 
-cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s) {
-    const cudaError_t e = launch_norm_c64(st, n, scratch, s);
+cudaError_t launch_renorm_c64(void* st, int n, void* scratch, bool summed, cudaStream_t s) {
+    const cudaError_t e = summed ? cudaSuccess : launch_norm_c64(st, n, scratch, s);
     if (e != cudaSuccess) return e;
     const uint64_t npairs = (1ull << n) / 2;
     const unsigned grid = (unsigned)(npairs < (uint64_t)RN_GRID * 256 ? (npairs + 255) / 256 : RN_GRID);
@@ -383,9 +344,9 @@ cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* part
                      : bitsums<double, float2, false>(p, n, sh.g, sh.nr, partials, out, nullptr, err, err_out, s);
 }
 
-cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, void* partials, void* out, const int* err,
-                                      int* err_out, cudaStream_t s) {
-    const cudaError_t e = launch_norm_c64(st, n, scratch, s);
+cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, bool summed, void* partials, void* out,
+                                      const int* err, int* err_out, cudaStream_t s) {
+    const cudaError_t e = summed ? cudaSuccess : launch_norm_c64(st, n, scratch, s);
     if (e != cudaSuccess) return e;
     const BitSumShape sh = bitsum_shape(n);
     return bitsums<double2, float2, true>((float2*)st, n, sh.g, sh.nr, partials, out,

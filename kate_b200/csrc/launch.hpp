@@ -66,8 +66,10 @@ struct Gate;
 std::string merge_gates_device(const std::vector<std::vector<Gate>>& blocks, int device, cudaStream_t stream,
                                std::vector<Gate>* out);
 cudaError_t launch_norm_c64(const void* st, int n, void* scratch, cudaStream_t s);  // ||psi||^2 only
-constexpr size_t renorm_result_offset() { return 148 * 4 * sizeof(double); }
-cudaError_t launch_renorm_c64(void* st, int n, void* scratch, cudaStream_t s);
+constexpr int RN_GRID = 148 * 4;  // CTAs at most
+constexpr size_t renorm_result_offset() { return RN_GRID * sizeof(double); }
+// summed: the pass before has left ||psi||^2 in the scratch (launch_block_c64).
+cudaError_t launch_renorm_c64(void* st, int n, void* scratch, bool summed, cudaStream_t s);
 
 // c128 state (double2 amplitudes)
 cudaError_t launch_set_basis0_c128(void* st, uint64_t dim, cudaStream_t s);
@@ -103,9 +105,10 @@ cudaError_t launch_tile_ws(void* st, const PassProg& prog, int* err, int grid, c
 
 // Complex64 pass of 5-qubit dense blocks on the tensor cores. from_zero: the
 // input is |0...0> and the state is not read. err: device int set to 1 if a
-// bounded wait gave up.
+// bounded wait gave up. norm: null, or the renormalisation scratch, which then
+// receives ||psi||^2 of the result.
 cudaError_t launch_block_c64(void* st, const BlockProg& prog, const void* bimg, bool from_zero, int* err, int grid,
-                             cudaStream_t s);
+                             void* norm, cudaStream_t s);
 int block_c64_grid(int n, int device);
 
 // Persistent batch kernel (k_batch.cu). head, done[circuits], zout (large
@@ -138,8 +141,8 @@ cudaError_t launch_bitsums(const void* st, int prec, int n, int kind, void* part
                            int* err_out, cudaStream_t s);
 // launch_renorm_c64 and the amplitude bit sums (kind 0) of the rescaled
 // state, which the rescaling pass adds up as it goes.
-cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, void* partials, void* out, const int* err,
-                                      int* err_out, cudaStream_t s);
+cudaError_t launch_renorm_bitsums_c64(void* st, int n, void* scratch, bool summed, void* partials, void* out,
+                                      const int* err, int* err_out, cudaStream_t s);
 // Amplitude bit sums of a complex128 state with an explicit shape: 2^g CTAs,
 // 2^nr rounds each (n = 12 + g + nr when n >= 12, nr <= 8). When g + nr > 0
 // the total out[0] is not written.

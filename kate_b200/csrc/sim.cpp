@@ -116,7 +116,9 @@ struct SimImpl {
     cudaError_t launch_pass(size_t i, cudaStream_t st) {
         if (small) return launch_small_range((int)i, (int)i + 1, 0, false, st);
         const PlannedPass& p = plan.passes[i];
-        if (p.bprog) return launch_block_c64(d_state, *p.bprog, d_bimg, i == 0 && zero_start, d_err, block_grid, st);
+        if (p.bprog)
+            return launch_block_c64(d_state, *p.bprog, d_bimg, i == 0 && zero_start, d_err, block_grid,
+                                    sum_norm && i + 1 == plan.passes.size() ? d_norm : nullptr, st);
         if (i == 0 && zero_start && jit_fn0) return jit_launch(jit_fn0, d_state, jit_mats[0], nullptr, jit_grid_n, st);
         if (i == 0 && prod_start && jit_fnP) return jit_launch(jit_fnP, d_state, jit_mats[0], &prod_tab, jit_grid_n, st);
         if (p.prog && i < jit_fn.size() && jit_fn[i]) return jit_launch(jit_fn[i], d_state, jit_mats[i], nullptr, jit_grid_n, st);
@@ -125,6 +127,9 @@ struct SimImpl {
         return launch_pass_generic(d_state, precision, hpasses[i], d_ops, d_pool, grid, st);
     }
     int block_grid = 0;
+    bool sum_norm = false;  // the pass being enqueued, if it is the last, leaves ||psi||^2 in d_norm
+    // Whether the last pass can: it is one of tensor-core blocks.
+    bool last_sums_norm() const { return !small && !plan.passes.empty() && plan.passes.back().bprog; }
     // Whether the first pass generates |0...0> itself.
     bool starts_from_zero() const { return jit_fn0 || (!plan.passes.empty() && plan.passes[0].bprog); }
 
@@ -579,16 +584,18 @@ std::string Simulator::enqueue_passes(void* stream, bool sums) {
     for (size_t i = 0; i < S.hpasses.size() && !S.small; i++) {
         S.zero_start = zs && i == 0;
         S.prod_start = ps && i == 0;
+        S.sum_norm = S.last_sums_norm();
         const cudaError_t ce = S.launch_pass(i, st);
-        S.zero_start = S.prod_start = false;
+        S.zero_start = S.prod_start = S.sum_norm = false;
         KCHECK(ce);
     }
     if (S.precision == 1) {
         // Complex64: ||psi|| in FP64, then the state rescaled to norm 1.
+        const bool summed = S.last_sums_norm();
         if (sums)
-            KCHECK(launch_renorm_bitsums_c64(S.d_state, S.n, S.d_norm, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
+            KCHECK(launch_renorm_bitsums_c64(S.d_state, S.n, S.d_norm, summed, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
         else
-            KCHECK(launch_renorm_c64(S.d_state, S.n, S.d_norm, st));
+            KCHECK(launch_renorm_c64(S.d_state, S.n, S.d_norm, summed, st));
         S.renormed = true;
     } else if (sums && !S.small) {
         KCHECK(launch_bitsums(S.d_state, 0, S.n, 0, S.d_part, S.res_sums(), S.d_err, S.res_flag(), st));
@@ -779,7 +786,8 @@ std::string Simulator::profile_passes(float* ms, float* init_ms) {
 
 int Simulator::launches_per_run() const {
     if (d_->small) return 1 + (d_->precision == 1 ? 2 : 0);
-    return (d_->starts_from_zero() ? 0 : 1) + (int)d_->hpasses.size() + (d_->precision == 1 ? 2 : 0);
+    return (d_->starts_from_zero() ? 0 : 1) + (int)d_->hpasses.size() +
+           (d_->precision == 1 ? d_->last_sums_norm() ? 1 : 2 : 0);
 }
 
 std::string Simulator::norm2_before_renorm(double* out) {
