@@ -225,8 +225,7 @@ KATE_API kate_status kate_sim_probabilities(kate_sim* s, double* out);
  * Sampled on the device (any qubit count): shot k draws u_k = (the k-th
  * splitmix64 output of `seed` >> 11) * 2^-53 and takes the first index whose
  * FP64 cumulative probability exceeds u_k times the total (indices of
- * probability 0 are never drawn); only the uniforms and the samples cross
- * PCIe. The reference has no sampling; its measurement is
+ * probability 0 are never drawn); only the samples cross PCIe. The reference has no sampling; its measurement is
  * HIPcode/simulator.hpp:483-543. */
 KATE_API kate_status kate_sim_sample(kate_sim* s, int shots, uint64_t seed, uint64_t* out);
 
@@ -247,8 +246,9 @@ KATE_API kate_status kate_sim_nqbits(kate_sim* s, int* out);
 KATE_API kate_status kate_sim_num_passes(kate_sim* s, int* out);
 KATE_API kate_status kate_sim_get_pass(kate_sim* s, int i, int* tile_qbits, int* m, int* ngates);
 /* Kernel that runs pass i of the simulator: 0 generic shared-memory
- * kernel, 1 register-staged interpreter, 2 pass-specialised kernel
- * (complex128; see kate_plan_pass_source), 3 complex64 tensor-core blocks.
+ * kernel, 1 register-staged interpreter (below 12 qubits one launch of it
+ * runs every pass), 2 pass-specialised kernel (complex128; see
+ * kate_plan_pass_source), 3 complex64 tensor-core blocks.
  * Replaces the choice executeCommand makes per group instruction
  * (HIPcode/simulator.hpp:760-810). */
 KATE_API kate_status kate_sim_pass_kernel(kate_sim* s, int i, int* kind);

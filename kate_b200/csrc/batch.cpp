@@ -399,9 +399,10 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
     // Cosets per pass task: at most `chunk`, and a level split into at most
     // `split` tasks: 16 when there are few circuits, so that a level spreads
     // over several CTAs, fewer when the circuits alone keep two waves of CTAs
-    // busy (300 resident CTAs): a task costs about 19 us beside its cosets'
-    // 4.7 us each (dequeuing, descriptors, operand images or tables, the
-    // dependency's round trip).
+    // busy (300 resident CTAs), since a task costs its operand images or
+    // tables and the dependency's round trip beside its cosets' 4.7 us each.
+    // With 300, 600, 900 and 1300 here 192 circuits of 10 to 20 qubits take
+    // 5.10, 5.15, 5.28 and 5.45 ms, 96 of 14 to 18 1.96, 1.68, 1.85 and 1.97.
     const uint32_t split = (uint32_t)std::min<size_t>(16, std::max<size_t>(1, 600 / std::max<size_t>(1, large.size())));
     auto pass_cosets = [&](const CircPack& P) -> uint32_t {
         const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS);
