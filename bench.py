@@ -212,14 +212,21 @@ def per_pass_gbs(alg_bytes, pass_ms, peak):
 PASS_KERNEL = "kate_pass (pass-specialised register-staged group pass, NVRTC for sm_100a)"
 
 
-def pass_roofline(n, npass, launches, ms_per_step, init_ms):
-    """Algorithmic bytes and time of a step's group passes. Every pass reads
-    and writes the 16-byte amplitudes once; when the run starts from |0..0>
-    the first pass generates its input (launches == passes: no separate
-    initialisation kernel) and only writes. Returns (bytes per launch on
-    average, ms per launch on average, achieved GB/s)."""
+def pass_roofline(n, passes, launches, ms_per_step, init_ms):
+    """Algorithmic bytes and time of a step's group passes (passes: the tile
+    qubits of each, and its gates). A pass reads and writes the 16-byte
+    amplitudes once, those in which every qubit that no tile up to its own
+    has held is |0>: the run starts from |0..0>, the others are zero and stay
+    so. When the first pass generates its input (launches == passes: no
+    separate initialisation kernel) it writes all amplitudes and reads none.
+    Returns (bytes per launch on average, ms per launch on average, achieved
+    GB/s)."""
+    npass = len(passes)
     zero_start = launches == npass
-    step_bytes = (2 * npass - (1 if zero_start else 0)) * 16.0 * 2 ** n
+    held, step_bytes = set(), 0.0
+    for i, (tile, _) in enumerate(passes):
+        held |= set(tile)
+        step_bytes += 16.0 * 2 ** n if zero_start and i == 0 else 2 * 16.0 * 2 ** len(held)
     step_ms = ms_per_step - (0.0 if zero_start else init_ms)
     return step_bytes / npass, step_ms / npass, step_bytes / (step_ms / 1000.0) / 1e9
 
@@ -483,7 +490,7 @@ def main():
 
     # Per-launch times of the group-pass kernel (events between launches).
     init_ms, pass_ms = sim.profile_passes()
-    alg_bytes, avg_pass_ms, achieved = pass_roofline(n, len(passes), launches, ms_per_step, init_ms)
+    alg_bytes, avg_pass_ms, achieved = pass_roofline(n, passes, launches, ms_per_step, init_ms)
     peak, peak_kind = measured_hbm_peak()
     sim_work = sim.pass_work()
     clk_summary = clk.summary()
@@ -796,7 +803,7 @@ def run_qulacs(args):
         ev1.synchronize()
     ms = ev0.elapsed_time(ev1) / args.steps
     init_ms, pass_ms = sim.profile_passes()
-    alg, avg_pass, _ = pass_roofline(n, len(passes), launches, ms, init_ms)
+    alg, avg_pass, _ = pass_roofline(n, passes, launches, ms, init_ms)
     peak, peak_kind = measured_hbm_peak()
     kate_proba = sim.execute().as_array()
     sim.close()

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <numeric>
 #include <atomic>
 #include <condition_variable>
@@ -469,6 +470,27 @@ DevPass to_devpass(int n, const PlannedPass& p, int op0) {
     return d;
 }
 
+// PlannedPass::idle of every pass, and the programs' coset bits in that order.
+// A pass moves qubits among its tile's physical bits only, so the bits that no
+// pass before has held are those of the qubits it has not.
+static void mark_idle(Plan& plan) {
+    uint64_t held = 0;
+    for (PlannedPass& pp : plan.passes) {
+        for (int b : pp.phys_in) held |= 1ull << b;
+        uint8_t order[48] = {0};
+        int k = 0;
+        for (int v = 0; v < 2; v++)  // those a pass before has held, then the idle ones
+            for (int b = 0; b < plan.n; b++)
+                if (std::find(pp.phys_in.begin(), pp.phys_in.end(), b) == pp.phys_in.end() &&
+                    (((held >> b) & 1ull) == 0) == (v == 1)) {
+                    order[k++] = (uint8_t)b;
+                    if (v == 1) pp.idle++;
+                }
+        if (pp.prog) std::memcpy(pp.prog->cphys, order, sizeof order);
+        if (pp.bprog) std::memcpy(pp.bprog->cphys, order, sizeof order);
+    }
+}
+
 void lower_pass(const Plan& plan, PlannedPass& pass, const std::vector<int>& phys, std::vector<Cx>& pool) {
     const int m = (int)pass.phys_in.size();
     auto tile_bit = [&](int q) -> int {
@@ -916,6 +938,7 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
       }
     }
     plan.final_phys = L.phys;
+    if (n > KATE_TILE_BITS) mark_idle(plan);
     return "";
 }
 

@@ -69,6 +69,11 @@ struct PlannedPass {
     std::shared_ptr<BlockProg> bprog;  // complex64 tensor-core block program, if it applies
     std::shared_ptr<PassProg> sprog;   // program of the one-CTA kernel (states of fewer than 12 qubits)
     std::string prog_note;           // why the generic kernel runs this pass, if it does
+    // Qubits outside the tile that no pass before has held; the programs list
+    // them last among the coset bits. In a run from |0...0> they are still
+    // |0>: only the first 2^(coset bits - idle) cosets are not zero, and a
+    // zero coset stays zero under any pass.
+    int idle = 0;
 };
 
 // FP64 instructions per amplitude that the pass-specialised kernel of a
