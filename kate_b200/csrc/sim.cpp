@@ -120,7 +120,7 @@ struct SimImpl {
         // Only the cosets that are not zero (a first pass that generates
         // |0...0> writes them all). A 30-qubit layered circuit reaches its
         // last qubits in the fourth of 20 passes, an SU(4) brickwork in
-        // complex64 in its eighth of 26: 200.8 -> 182.4 and 94.4 -> 73.5 ms a
+        // complex64 in its ninth of 26: 200.8 -> 182.4 and 94.4 -> 73.5 ms a
         // run; 23 qubits in three passes 396 -> 263 us.
         const int idle = basis0 && !(i == 0 && zero_start) ? p.idle : 0;
         if (p.bprog) {
