@@ -117,6 +117,8 @@ std::string pack_circuit(const Program& in, const BatchTune& tune, bool resident
         header(&pp, bp);
         if (bp.m != KATE_TILE_BITS) return "internal: batch pass tile is not 12 qubits";
         if (!out.small && bp.tphys[0] != 0) return "internal: batch pass tile does not hold physical bit 0";
+        if (pp.prog) std::memcpy(bp.cphys, pp.prog->cphys, 48);
+        out.ncos.push_back((1u << bp.ncb) >> (!out.progs.empty() && (pp.prog || pp.bprog) ? pp.idle : 0));
         if (out.blocks) {
             BlockProg b = *pp.bprog;
             const uint64_t at = put_bytes(out.blob, &b, sizeof(BlockProg));
@@ -150,6 +152,7 @@ std::string pack_circuit(const Program& in, const BatchTune& tune, bool resident
     if (out.progs.empty() && !out.small) {
         BatchProg bp{};
         header(nullptr, bp);
+        out.ncos.push_back(1u << bp.ncb);
         out.progs.push_back(bp);
     }
     // Register-staged programs carry their own matrices; only shared-memory
@@ -409,15 +412,17 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
         return std::max<uint32_t>(1, std::min<uint32_t>(chunk, ncos / split));
     };
     auto pass_tasks = [&](const CircPack& P) -> uint64_t {
-        const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS), cch = pass_cosets(P);
-        return (ncos + cch - 1) / cch;
+        const uint32_t cch = pass_cosets(P);
+        uint64_t tasks = 0;
+        for (uint32_t ncos : P.ncos) tasks += (ncos + cch - 1) / cch;
+        return tasks;
     };
     auto zred_tasks = [&](const CircPack& P) -> uint64_t {
         const uint64_t nch = std::max<uint64_t>(1, (1ull << P.n_sim) >> 16);
         return (nch + zchunks - 1) / zchunks;
     };
     uint64_t L = 0;
-    for (int ci : large) L += pass_tasks(packs[ci]) * packs[ci].progs.size() + zred_tasks(packs[ci]);
+    for (int ci : large) L += pass_tasks(packs[ci]) + zred_tasks(packs[ci]);
     const uint64_t Sn = small.size();
     if (L + Sn > (uint64_t)INT32_MAX) return fail("too many tasks");
     S->tasks.reserve(L + Sn);
@@ -476,7 +481,7 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
                 const size_t nprog = P.progs.size();
                 const int before = need[k];
                 if (lev < nprog) {
-                    const uint32_t ncos = 1u << (P.n_sim - KATE_TILE_BITS);
+                    const uint32_t ncos = P.ncos[lev];
                     const uint32_t cch = pass_cosets(P);
                     for (uint32_t c0 = 0; c0 < ncos; c0 += cch) {
                         BatchTask t{};

@@ -47,6 +47,8 @@ struct CircPack {
     bool small = false;  // runs whole in one CTA's shared memory (BT_SMALL)
     std::vector<uint8_t> zbit;     // output x reads this bit of the final layout
     std::vector<BatchProg> progs;  // one per pass
+    std::vector<uint32_t> ncos;    // cosets each pass visits: the first all, the others those of qubits
+                                   // that a pass before has held (PlannedPass::idle; the rest are zero)
     std::vector<uint8_t> blob;
     std::vector<DevOp> sops;
     std::vector<Cx> pool;

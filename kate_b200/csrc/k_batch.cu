@@ -618,7 +618,8 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
                 }
                 if (t == TAKER && s + 1 == nsteps) fetch_task(take_index(), now ^ 1u);
                 __syncthreads();
-                run_any(T, P, blob, tbc, tilec, cbase, sops, pool, t);
+                // A first pass's other cosets are zero in and out.
+                if (!K.first || cbase == 0) run_any(T, P, blob, tbc, tilec, cbase, sops, pool, t);
                 if (!small) {
                     __syncthreads();
                     store_tile<C2, true>(T, st, c, tbc, t);

@@ -147,6 +147,7 @@ struct Req {
     uint64_t state_off = 0, aux_off = 0;
     int64_t prog0 = 0, zoff = 0, poff = 0, uoff = 0, soff = 0;
     uint32_t ncos = 1, nch = 1;
+    std::vector<uint32_t> pass_ncos;  // CircPack::ncos
     int npass = 0, levels = 0, next_level = 0;
     BatchCirc circ{};
 };
@@ -244,6 +245,7 @@ struct ServerImpl {
         const int n = P.n_sim;
         const uint64_t sbytes = (1ull << n) * amp_bytes();
         r->ncos = 1u << (n - KATE_TILE_BITS);
+        r->pass_ncos = P.ncos;
         r->nch = (uint32_t)std::max<uint64_t>(1, (1ull << n) >> 16);
         // Section sizes with worst-case padding for element alignment.
         const uint64_t need = P.progs.size() * sizeof(BatchProg) + P.blob.size() + P.sops.size() * sizeof(DevOp) +
@@ -344,7 +346,7 @@ struct ServerImpl {
     double level_latency_us(const Req* r, int a) const {
         if (a < r->npass) {
             const uint32_t ch = pass_cosets(r);
-            const uint64_t tasks = (r->ncos + ch - 1) / ch;
+            const uint64_t tasks = (r->pass_ncos[a] + ch - 1) / ch;
             const uint64_t waves = (tasks + grid - 1) / std::max(1, grid);
             return (double)waves * (20.0 * ch + 5.0);
         }
@@ -355,7 +357,7 @@ struct ServerImpl {
 
     // Cost of level a of r in tile passes (for the step budget).
     int64_t level_cost(const Req* r, int a) const {
-        if (a < r->npass) return r->ncos;
+        if (a < r->npass) return r->pass_ncos[a];
         if (a == r->npass) return std::max<int64_t>(1, r->ncos / 2);
         if (a == r->npass + 1) return 1;
         return std::max<int64_t>(1, r->ncos / 4);
@@ -485,7 +487,8 @@ struct ServerImpl {
             };
             if (a < r->npass) {
                 const uint32_t ch = pass_cosets(r);
-                for (uint32_t c0 = 0; c0 < r->ncos; c0 += ch) add(BT_PASS, c0, std::min(r->ncos, c0 + ch));
+                const uint32_t nc = r->pass_ncos[a];
+                for (uint32_t c0 = 0; c0 < nc; c0 += ch) add(BT_PASS, c0, std::min(nc, c0 + ch));
             } else if (a == r->npass) {
                 for (uint32_t c0 = 0; c0 < r->nch; c0 += zch) add(BT_ZRED, c0, std::min(r->nch, c0 + zch));
             } else if (a == r->npass + 1) {

@@ -3,13 +3,14 @@ are zero); runs from a product state skip nothing. Circuits that leave qubits
 out, reach them late or take them in any order, on every kernel, against the
 oracle, with both starts on one simulator so that the buffer holds an old
 state."""
+import ctypes
 import os
 
 import numpy as np
 import pytest
 
 import kate_b200 as K
-from kate_b200 import circuits
+from kate_b200 import _lib, circuits
 from common import haar, random_circuit
 
 pytestmark = pytest.mark.gpu
@@ -71,3 +72,21 @@ def test_complex64(n, oracle):
             sim.execute()
             assert np.abs(sim.state() - ref).max() <= 1e-4, name
         sim.close()
+
+
+@pytest.mark.parametrize("prec,blocks,tol", [(K.C128, 0, 1e-12), (K.C64, 0, 2e-5), (K.C64, 1, 2e-5)])
+def test_batch(oracle, prec, blocks, tol):
+    # Bars as for the batch engine; two runs, so that the arena holds old states.
+    specs = [(n, g) for n in (13, 16, 18) for g in (late(n, n), late(n - 2, n + 1), circuits.hea(n, n, seed=n), [])]
+    opts = _lib.BatchOptions()
+    _lib.lib().kate_batch_options_default(ctypes.byref(opts))
+    for n, _ in specs:
+        opts.tune[n].blocks = blocks
+    b = K.Batch([K.Circuit(n, g) for n, g in specs], precision=prec, options=opts)
+    for _ in range(2):
+        b.run()
+        for (n, g), z in zip(specs, b.expect_z()):
+            p = np.abs(oracle.simulate(n, g)) ** 2
+            x = np.arange(1 << n)
+            want = [p[(x >> q) & 1 == 0].sum() - p[(x >> q) & 1 == 1].sum() for q in range(n)]
+            assert np.abs(z - want).max() <= tol, (n, len(g))
