@@ -281,6 +281,8 @@ KATE_API kate_status kate_sim_norm2_before_renorm(kate_sim* s, double* norm2);
 #define KATE_PLAN_REMAP_SEARCH 16u /* choose the qubits moved into the low bits by trying every subset
                                       of the tile, and the gate cap per pass among 96..144 (fewest
                                       passes): what complex128 simulators do */
+#define KATE_PLAN_SIMULATOR 32u /* the plan a simulator of the circuit makes (a complex64 one with KATE_PLAN_C64);
+                                   max_tile, coalesce and the other flags are not looked at */
 KATE_API kate_status kate_plan_create(const kate_circuit* c, int max_tile, int coalesce, unsigned flags,
                                       kate_plan** out);
 KATE_API kate_status kate_plan_destroy(kate_plan* p);
@@ -295,7 +297,9 @@ KATE_API kate_status kate_plan_num_ops(const kate_plan* p, int* out);
 KATE_API kate_status kate_plan_get_op(const kate_plan* p, int i, int* ints, uint64_t* pmask, double* vals);
 /* Register-staged program of pass i (the PassProg struct of
  * kate_b200/csrc/device_types.h, *size bytes, copied when cap allows);
- * *has = 0 when the pass runs on the generic shared-memory kernel. */
+ * *has = 0 when the pass runs on the generic shared-memory kernel. In a
+ * KATE_PLAN_SIMULATOR plan of fewer than 12 qubits: the program of the
+ * one-launch kernel, and 0 for every pass when that does not take them all. */
 KATE_API kate_status kate_plan_get_program(const kate_plan* p, int i, void* out, size_t cap, size_t* size, int* has);
 KATE_API kate_status kate_plan_num_smem_ops(const kate_plan* p, int* out);
 /* CUDA source of the pass-specialised kernel of pass i: its register-staged

@@ -616,6 +616,7 @@ kate_status kate_plan_create(const kate_circuit* c, int max_tile, int coalesce, 
         opt.fuse_1q = !(flags & KATE_PLAN_NO_FUSE1Q);
         opt.c64 = (flags & KATE_PLAN_C64) != 0;
         opt.dense2_reg = !opt.c64 && !(flags & KATE_PLAN_NO_DENSE2);
+        if (flags & KATE_PLAN_SIMULATOR) opt = kate::simulator_plan_options(prog.nqbits, opt.c64 ? 1 : 0);
         auto* p = new kate_plan();
         std::string e = kate::build_plan(prog, opt, &p->plan);
         if (!e.empty()) {
@@ -698,8 +699,9 @@ kate_status kate_plan_get_program(const kate_plan* p, int i, void* out, size_t c
     REQUIRE(i >= 0 && i < (int)p->plan.passes.size(), "pass index out of range");
     *size = sizeof(PassProg);
     const auto& pp = p->plan.passes[i];
-    *has = pp.prog ? 1 : 0;
-    if (pp.prog && out && cap >= sizeof(PassProg)) std::memcpy(out, pp.prog.get(), sizeof(PassProg));
+    const PassProg* prog = pp.prog ? pp.prog.get() : pp.sprog.get();
+    *has = prog ? 1 : 0;
+    if (prog && out && cap >= sizeof(PassProg)) std::memcpy(out, prog, sizeof(PassProg));
     return KATE_OK;
 }
 

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <numeric>
 #include <atomic>
@@ -602,6 +603,50 @@ std::vector<PlannedPass> plan_relayout(int n, const std::vector<int>& phys0, con
     return out;
 }
 
+PlanOptions simulator_plan_options(int n, int precision) {
+    PlanOptions o;
+    o.c64 = precision == 1;
+    o.lower_all = false;
+    {
+        // Dense two-qubit gates as register ops for complex128, where the
+        // pass-specialised kernels run them straight-line.
+        const char* jv = std::getenv("KATE_JIT");
+        o.dense2_reg = precision == 0 && !(jv && std::atoi(jv) == 0);
+    }
+    if (n < KATE_TILE_BITS) {
+        // The whole state is one tile: nothing to remap between passes, and
+        // the one-CTA kernel computes in FP64 for both precisions.
+        o.small = true;
+        o.max_gates_per_pass = 64;  // two register bits: up to 40 stages
+        o.remap = false;
+        o.c64 = false;
+        o.dense2_reg = true;
+    }
+    // Complex128 passes of 27 qubits and more choose the qubits they move
+    // into the low bits by trying every subset, and the gate cap per pass
+    // among a few (about 15 ms of planning for a 30-qubit, 1780-gate
+    // circuit; below 27 qubits a pass takes under 0.7 ms and the search
+    // would cost more host time than it saves). KATE_REMAP_SEARCH=0 or 1
+    // forces it off or on.
+    {
+        const char* rs = std::getenv("KATE_REMAP_SEARCH");
+        const bool on = rs ? std::atoi(rs) != 0 : n >= 27;
+        o.remap_search = precision == 0 && on;
+        o.cap_search = o.remap_search;
+    }
+    // Contiguous low physical bits every tile holds (runs of 2^c amplitudes per access).
+    if (const char* e = std::getenv("KATE_COALESCE")) {
+        const int v = std::atoi(e);
+        if (v >= 1 && v <= 8) o.coalesce = v;
+    }
+    // Gates a pass may take at most (the planner packs greedily up to it).
+    if (const char* e = std::getenv("KATE_MAX_GATES")) {
+        const int v = std::atoi(e);
+        if (v >= 1 && v <= 160) o.max_gates_per_pass = v, o.cap_search = false;
+    }
+    return o;
+}
+
 std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
     if (opt.cap_search && !opt.c64) {
         // One plan per cap, on its own thread.
@@ -939,6 +984,15 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
     }
     plan.final_phys = L.phys;
     if (n > KATE_TILE_BITS) mark_idle(plan);
+    // The one-CTA kernel runs a plan's programs in one launch: when a pass has
+    // none (eight generic 5-qubit diagonals are more ops than a program
+    // holds), the generic kernel runs them all.
+    if (opt.small &&
+        std::any_of(plan.passes.begin(), plan.passes.end(), [](const PlannedPass& p) { return !p.sprog; }))
+        for (PlannedPass& pp : plan.passes) {
+            pp.sprog.reset();
+            if (pp.ops.empty()) lower_pass(plan, pp, pp.phys_before, plan.pool);
+        }
     return "";
 }
 

@@ -67,7 +67,8 @@ struct PlannedPass {
     std::vector<int> phys_before;  // layout (logical -> physical) when the pass starts
     std::shared_ptr<PassProg> prog;  // register-staged program (tile kernel), if it applies
     std::shared_ptr<BlockProg> bprog;  // complex64 tensor-core block program, if it applies
-    std::shared_ptr<PassProg> sprog;   // program of the one-CTA kernel (states of fewer than 12 qubits)
+    std::shared_ptr<PassProg> sprog;   // program of the one-CTA kernel (states of fewer than 12 qubits):
+                                       // every pass of a plan has one, or none has
     std::string prog_note;           // why the generic kernel runs this pass, if it does
     // Qubits outside the tile that no pass before has held; the programs list
     // them last among the coset bits. In a run from |0...0> they are still
@@ -105,6 +106,10 @@ struct Plan {
     std::vector<DevOp> smem_ops;     // shared-memory ops referenced by register-staged programs
     std::vector<uint8_t> bimg;       // complex64 block operand images (KATE_BLOCK_IMG_BYTES each)
 };
+
+// The options a simulator of n qubits plans with (precision 0: complex128, 1:
+// complex64; see the environment variables in the definition).
+PlanOptions simulator_plan_options(int n, int precision);
 
 // Classifies gates, plans passes and lowers them to device ops. Dense gates
 // above 5 qubits are rejected (message returned).

@@ -265,45 +265,7 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
         std::string e = pass_compile_default(impl->prog, 0, impl->prog.nqbits);
         if (!e.empty()) return fail(e);
     }
-    impl->opt.c64 = precision == 1;
-    impl->opt.lower_all = false;
-    {
-        // Dense two-qubit gates as register ops for complex128, where the
-        // pass-specialised kernels run them straight-line.
-        const char* jv = std::getenv("KATE_JIT");
-        impl->opt.dense2_reg = precision == 0 && !(jv && std::atoi(jv) == 0);
-    }
-    if (impl->n < KATE_TILE_BITS) {
-        // The whole state is one tile: nothing to remap between passes, and
-        // the one-CTA kernel computes in FP64 for both precisions.
-        impl->opt.small = true;
-        impl->opt.max_gates_per_pass = 64;  // two register bits: up to 40 stages
-        impl->opt.remap = false;
-        impl->opt.c64 = false;
-        impl->opt.dense2_reg = true;
-    }
-    // Complex128 passes of 27 qubits and more choose the qubits they move
-    // into the low bits by trying every subset, and the gate cap per pass
-    // among a few (about 15 ms of planning for a 30-qubit, 1780-gate
-    // circuit; below 27 qubits a pass takes under 0.7 ms and the search
-    // would cost more host time than it saves). KATE_REMAP_SEARCH=0 or 1
-    // forces it off or on.
-    {
-        const char* rs = std::getenv("KATE_REMAP_SEARCH");
-        const bool on = rs ? std::atoi(rs) != 0 : prog_in.nqbits >= 27;
-        impl->opt.remap_search = precision == 0 && on;
-        impl->opt.cap_search = impl->opt.remap_search;
-    }
-    // Contiguous low physical bits every tile holds (runs of 2^c amplitudes per access).
-    if (const char* e = std::getenv("KATE_COALESCE")) {
-        const int v = std::atoi(e);
-        if (v >= 1 && v <= 8) impl->opt.coalesce = v;
-    }
-    // Gates a pass may take at most (the planner packs greedily up to it).
-    if (const char* e = std::getenv("KATE_MAX_GATES")) {
-        const int v = std::atoi(e);
-        if (v >= 1 && v <= 160) impl->opt.max_gates_per_pass = v, impl->opt.cap_search = false;
-    }
+    impl->opt = simulator_plan_options(impl->n, precision);
     std::string e = build_plan(impl->prog, impl->opt, &impl->plan);
     if (!e.empty()) return fail(e);
 
@@ -333,6 +295,9 @@ std::string Simulator::create(const Program& prog_in, int precision, int device,
     const size_t o_bimg = put(impl->plan.bimg.data(), impl->plan.bimg.size());
     impl->small = impl->n < KATE_TILE_BITS;
     for (const auto& p : impl->plan.passes) impl->small = impl->small && p.sprog;
+    for (const auto& p : impl->plan.passes)
+        if (!p.prog && !p.bprog && !impl->small && p.ops.size() != p.gates.size())
+            return fail("internal: a pass has neither a program nor its device ops");
     size_t o_small = 0;
     if (impl->small) {
         const std::vector<char> blob = impl->small_blob();
