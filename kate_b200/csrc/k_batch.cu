@@ -94,10 +94,10 @@ constexpr uint32_t BLK_PROG = (sizeof(BlockProg) + 15) & ~15u;
 constexpr uint32_t BLK_REGION = 1024 + BLK_IMG + BLK_PROG;
 static_assert(sizeof(BlockProg) % 8 == 0, "BlockProg is copied as 8-byte words");
 // Per CTA, for the whole launch (complex64 batches with block programs):
-// the products' mbarrier and its phase, the TMEM columns, the wait flag.
-__shared__ uint64_t blk_mbar[2], blk_mbar_img;  // products' mbarrier of each group
+// the groups' words and their mbarriers' phases, the TMEM columns.
+__shared__ blk::GroupSync blk_group[2];
+__shared__ uint64_t blk_mbar_img;
 __shared__ uint32_t blk_tmem, blk_phase[2], blk_phase_img;
-__shared__ int blk_abort;
 
 // Waits (time-bounded) until `need` tasks of the circuit have finished; every
 // thread returns the same answer, after a barrier. *abort (shared) is set
@@ -174,8 +174,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     const uint32_t t = threadIdx.x, grp = t / G;
     const uint32_t c0 = K.c0, c1 = K.c1;
     const bool first = K.first != 0;
-    const uint32_t tmem = blk_tmem + grp * blk::TMEM_COLS, mbar = blk::smem_u32(&blk_mbar[grp]);
-    int* abort_flag = &blk_abort;
+    const uint32_t tmem = blk_tmem + grp * blk::TMEM_COLS, sync = blk::smem_u32(&blk_group[grp]);
     uint32_t phase = blk_phase[grp];  // every thread of the group keeps the same copy; its first one stores it back
     unsigned char* raw = batch_smem_raw + 2 * TS * sizeof(float2);
     const uint32_t rawa = blk::smem_u32(raw);
@@ -191,7 +190,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
     uint32_t phase_img = blk_phase_img;
     const bool img_ok = blk::load_images(P.nblocks, [&](int b) { return src + P.bimg[b]; }, bbase,
                                          blk::smem_u32(&blk_mbar_img), phase_img);
-    if (!img_ok) *abort_flag = 1;
+    if (!img_ok) blk_group[0].gave_up = blk_group[1].gave_up = 1;  // before wait_dep's barrier
     blk::Pass<G> X;
     blk::setup(P, X);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -222,7 +221,7 @@ __device__ __noinline__ bool block_task(float2* st, const BatchProg& BP, const u
         }
         if (take) fetch_task(next, slot ^ 1u);
         blk::group_bar<G>();
-        ok = blk::apply_blocks(P, X, S, bbase, tmem, mbar, phase, abort_flag);
+        ok = blk::apply_blocks(P, X, S, bbase, tmem, sync, phase);
         if (!ok) break;
         blk::store_tile<true, false>(P, X, st, cb, S, unused);
         blk::group_bar<G>();
@@ -532,11 +531,11 @@ __global__ void __launch_bounds__(NT, sizeof(C2) == 8 ? 2 : 1)
     if constexpr (TB) {
         {
             if (t == 0) {
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar[0])) : "memory");
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar[1])) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_group[0].mbar)) : "memory");
+                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_group[1].mbar)) : "memory");
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(blk::smem_u32(&blk_mbar_img)) : "memory");
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-                blk_abort = 0;
+                blk_group[0].gave_up = blk_group[1].gave_up = 0;
                 blk_phase[0] = blk_phase[1] = 0;
                 blk_phase_img = 0;
             }

@@ -43,7 +43,10 @@ constexpr uint32_t S_BYTES = TS * 8;  // one staging tile (float2)
 // operand's hi and lo parts (128 lanes x 64 BF16 = 32 columns each).
 constexpr uint32_t TMEM_COLS = 128;
 constexpr uint32_t TM_AHI = 64, TM_ALO = 96;
-constexpr long WAIT_LIMIT = 1L << 24;
+#ifndef KATE_BLOCK_WAIT_LIMIT
+#define KATE_BLOCK_WAIT_LIMIT (1L << 24)
+#endif
+constexpr long WAIT_LIMIT = KATE_BLOCK_WAIT_LIMIT;  // polls of an mbarrier before a wait gives up
 // The pass's staging-tile swizzle (BlockProg::smask, chosen on the host):
 // element e sits at e ^ sum_k parity(e & f[k]) << k. Linear over GF(2), so
 // offsets of XOR-combined indices XOR.
@@ -160,6 +163,21 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
     }
 }
+
+// A group's words in shared memory: the mbarrier of its products, and whether
+// a wait of its threads gave up. Threads of other groups touch neither while
+// the group works: between the barrier that ends a block, after which the
+// group's threads read the flag, and the next block's products, before which
+// none of them can set it, lies another barrier of the group, so all of them
+// read the same. (The groups of a CTA have no barrier in common. With one flag
+// for both, a thread could see the other group's where its neighbours did not
+// yet, and they would wait for one another at different barriers, without a
+// bound.)
+struct GroupSync {
+    uint64_t mbar;
+    int gave_up, pad;
+};
+constexpr uint32_t GAVE_UP = 8;  // its offset
 
 // Barrier of the G threads that work on one tile: the CTA, or named barrier
 // 1 + (the group's index).
@@ -309,12 +327,12 @@ __device__ __forceinline__ void zero_tile(float2* S, bool one) {
 // Applies the pass's blocks to the staging tile S (its copy complete and
 // visible to every thread of the group), in the 128 TMEM columns from tmem
 // (accumulator, then the A parts). B images at shared address bimg (block b
-// at bimg + b * KATE_BLOCK_IMG_BYTES, 1024-byte aligned). Returns false when
-// a product wait gave up (after every thread of the group has left the block
-// loop).
+// at bimg + b * KATE_BLOCK_IMG_BYTES, 1024-byte aligned). sync: shared address
+// of the group's GroupSync. Returns false, to every thread of the group, when
+// one of its waits for the products gave up.
 template <int G>
 __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& X, float2* S, uint32_t bimg,
-                                             uint32_t tmem, uint32_t mbar, uint32_t& phase, int* abort_flag) {
+                                             uint32_t tmem, uint32_t sync, uint32_t& phase) {
     const uint32_t t = threadIdx.x & (uint32_t)(G - 1);
     const uint32_t lanes = tmem + (((threadIdx.x >> 5) & 3u) << 21);  // this warp's 32 lanes
     constexpr uint32_t NH = NT / G;                                   // K halves per thread
@@ -366,15 +384,15 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& 
                 mma_bf16_ts(tmem, tmem + TM_AHI + kc, b_lo, 1u);
                 mma_bf16_ts(tmem, tmem + TM_ALO + kc, b_hi, 1u);
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(sync)
                          : "memory");
         }
         // Every thread waits for the products itself (try_wait suspends the
         // waiting thread), so no barrier sits between the products and the
         // read-back. A wait that gives up raises the flag; the read-back
         // still runs (its values are then unused) so that every thread
-        // reaches the barrier below, after which all see the flag.
-        if (!mbar_wait(mbar, phase)) *abort_flag = 1;
+        // reaches the barrier below, after which the group sees the flag.
+        if (!mbar_wait(sync, phase)) asm volatile("st.shared.u32 [%0], 1;" ::"r"(sync + GAVE_UP) : "memory");
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // 3. Results: row t & 127, block indices 16h..16h+15 in columns
@@ -409,7 +427,12 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& 
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         group_bar<G>();
-        if (*abort_flag) return false;
+        uint32_t stop;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(stop) : "r"(sync + GAVE_UP) : "memory");
+        // The vote tells the compiler that the branch is the same for the
+        // warp; without it the loops around lose their uniform registers and
+        // spill.
+        if (__any_sync(0xffffffffu, stop != 0)) return false;
     }
     return true;
 }

@@ -36,7 +36,7 @@ using namespace blk;
 constexpr int G = 128, NG = NT / G;                                             // groups per CTA
 constexpr uint32_t OFF_B = 0;                                                   // blocks' B images
 constexpr uint32_t OFF_S = OFF_B + KATE_C64_MAX_BLOCKS * KATE_BLOCK_IMG_BYTES;  // a staging tile per group
-constexpr uint32_t OFF_MISC = OFF_S + NG * S_BYTES;  // groups' mbarriers, images' mbarrier, TMEM slot, abort flag
+constexpr uint32_t OFF_MISC = OFF_S + NG * S_BYTES;  // groups' words, images' mbarrier, TMEM slot
 constexpr uint32_t SMEM_BYTES = OFF_MISC + 64 + 1024;  // + alignment slack
 
 template <bool NORM>
@@ -49,14 +49,15 @@ __global__ void __launch_bounds__(NT, 2)
     const uint32_t base = (raw + 1023u) & ~1023u;  // 1024-byte aligned operand region
     uint8_t* gbase = smem_raw + (base - raw);
     const uint32_t t = threadIdx.x, grp = t / G;
-    const uint32_t mbar = base + OFF_MISC + 8u * grp, mbar_img = base + OFF_MISC + 8u * NG;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + OFF_MISC + 8 * NG + 8);
-    int* abort_flag = reinterpret_cast<int*>(gbase + OFF_MISC + 8 * NG + 16);
+    constexpr uint32_t GS = sizeof(GroupSync);
+    GroupSync* groups = reinterpret_cast<GroupSync*>(gbase + OFF_MISC);
+    const uint32_t sync = base + OFF_MISC + GS * grp, mbar_img = base + OFF_MISC + GS * NG;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + OFF_MISC + GS * NG + 8);
     if (t == 0) {
         for (int i = 0; i <= NG; i++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + OFF_MISC + 8u * i) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(base + OFF_MISC + GS * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        *abort_flag = 0;
+        for (int i = 0; i < NG; i++) groups[i].gave_up = 0;
     }
     tmem_alloc(tmem_slot, NG * TMEM_COLS);
     __syncthreads();
@@ -64,7 +65,7 @@ __global__ void __launch_bounds__(NT, 2)
     uint32_t phase_img = 0;
     if (!load_images(P.nblocks, [&](int b) { return bimg + P.bimg[b]; }, base + OFF_B, mbar_img, phase_img) &&
         t == 0)
-        *abort_flag = 1;
+        for (int i = 0; i < NG; i++) groups[i].gave_up = 1;
     Pass<G> X;
     setup(P, X);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -91,11 +92,11 @@ __global__ void __launch_bounds__(NT, 2)
             asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
         }
         group_bar<G>();
-        if (!apply_blocks(P, X, S, base + OFF_B, tmem, mbar, phase, abort_flag)) break;
+        if (!apply_blocks(P, X, S, base + OFF_B, tmem, sync, phase)) break;
         store_tile<false, NORM>(P, X, st, cb, S, norm);
         group_bar<G>();
     }
-    if (*abort_flag && t == 0) atomicExch(err, 1);
+    if (groups[grp].gave_up && t % G == 0) atomicExch(err, 1);
     tmem_free(*tmem_slot, NG * TMEM_COLS);
     if constexpr (NORM) finish_norm<NT>(norm, N);
 }
