@@ -48,8 +48,10 @@ __device__ __forceinline__ void prefetch(SmallTables& T, const BatchProg& P, con
     copy16(T.stab, blob + P.stab_off, (P.nstages * 88 + 15) & ~15, t, nt);
 }
 
-// m: the programs' tile bits; 2^m / N threads run them. With fewer than 32 of these the warp's other lanes repeat them (the same values
-// to the same places), so that every lane takes every barrier.
+// m: the programs' tile bits; 2^m / N threads run them. With fewer than 32 of
+// these the warp's other lanes repeat them, so that every lane takes every
+// barrier: the same values to the same places, since a stage stores only once
+// the whole warp has loaded (run_program).
 // init: 0 the state as it is, 1 |0...0>, 2 the product state PI.
 // SM: whether a program has shared-memory ops (without them the program loop
 // makes no call, and nothing is kept in memory around one).

@@ -604,6 +604,10 @@ __device__ __forceinline__ void run_program(const TT& T, int nops, uint32_t tb, 
         }
         const uint16_t* tab = T.stab[si];
         const uint32_t v0 = tab[36], v1 = tab[37], v2 = tab[38], v3 = tab[39];
+        // With fewer threads than a warp its other lanes repeat them
+        // (k_small.cu): a lane stores over what the one that repeats it has
+        // to have loaded, whatever way the ops between took each of them.
+        if constexpr (N < 16) __syncwarp();
 #pragma unroll
         for (int j = 0; j < N; j++) A::sts(tb + reg_off(j, s0s, v0, v1, v2, v3), a[j]);
     };
