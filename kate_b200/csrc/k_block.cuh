@@ -2,9 +2,9 @@
 // pass kernel (k_block_c64.cu) and the batch kernel's block tasks
 // (k_batch.cu). A pass applies up to KATE_C64_MAX_BLOCKS dense 5-qubit blocks
 // (BlockProg, device_types.h) to 4096-amplitude coset tiles staged in shared
-// memory. A group of G threads works on a tile (128 in the simulator's pass
-// kernel, two groups per CTA; the whole CTA, 256, in the batch kernel, whose
-// tasks can be a single tile); per block:
+// memory. A group of G threads works on a tile (128, two groups per CTA, in
+// the simulator's pass kernel and in the batch kernel's tasks of two tiles and
+// more; the whole CTA, 256, in its tasks of a single tile); per block:
 //   1. every thread builds its part of the MMA A operand from the staging
 //      tile: row r = t & 127 (the values of the 7 non-block tile bits), all
 //      32 block indices or (G = 256) the 16 of K half t >> 7, re/im
@@ -166,13 +166,13 @@ __device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
 
 // A group's words in shared memory: the mbarrier of its products, and whether
 // a wait of its threads gave up. Threads of other groups touch neither while
-// the group works: between the barrier that ends a block, after which the
-// group's threads read the flag, and the next block's products, before which
-// none of them can set it, lies another barrier of the group, so all of them
-// read the same. (The groups of a CTA have no barrier in common. With one flag
-// for both, a thread could see the other group's where its neighbours did not
-// yet, and they would wait for one another at different barriers, without a
-// bound.)
+// the group works: between the barrier that ends a tile's last block, after
+// which the group's threads read the flag, and the next tile's products,
+// before which none of them can set it, lies another barrier of the group, so
+// all of them read the same. (The groups of a CTA have no barrier in common.
+// With one flag for both, a thread could see the other group's where its
+// neighbours did not yet, and they would wait for one another at different
+// barriers, without a bound.)
 struct GroupSync {
     uint64_t mbar;
     int gave_up, pad;
@@ -329,7 +329,7 @@ __device__ __forceinline__ void zero_tile(float2* S, bool one) {
 // (accumulator, then the A parts). B images at shared address bimg (block b
 // at bimg + b * KATE_BLOCK_IMG_BYTES, 1024-byte aligned). sync: shared address
 // of the group's GroupSync. Returns false, to every thread of the group, when
-// one of its waits for the products gave up.
+// one of its waits for the products gave up; the tile is then undefined.
 template <int G>
 __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& X, float2* S, uint32_t bimg,
                                              uint32_t tmem, uint32_t sync, uint32_t& phase) {
@@ -389,9 +389,9 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& 
         }
         // Every thread waits for the products itself (try_wait suspends the
         // waiting thread), so no barrier sits between the products and the
-        // read-back. A wait that gives up raises the flag; the read-back
-        // still runs (its values are then unused) so that every thread
-        // reaches the barrier below, after which the group sees the flag.
+        // read-back. A wait that gives up raises the flag; the read-back and
+        // the next block still run (their values are then unused), so that
+        // every thread takes the same barriers to the look at the flag.
         if (!mbar_wait(sync, phase)) asm volatile("st.shared.u32 [%0], 1;" ::"r"(sync + GAVE_UP) : "memory");
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -427,14 +427,13 @@ __device__ __forceinline__ bool apply_blocks(const BlockProg& P, const Pass<G>& 
         }
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         group_bar<G>();
-        uint32_t stop;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(stop) : "r"(sync + GAVE_UP) : "memory");
-        // The vote tells the compiler that the branch is the same for the
-        // warp; without it the loops around lose their uniform registers and
-        // spill.
-        if (__any_sync(0xffffffffu, stop != 0)) return false;
     }
-    return true;
+    // Once per tile (once per block, the look took 30 ns of each). The vote
+    // tells the compiler that the answer is the same for the warp; without it
+    // the loop over tiles loses its uniform registers and spills.
+    uint32_t stop;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(stop) : "r"(sync + GAVE_UP) : "memory");
+    return !__any_sync(0xffffffffu, stop != 0);
 }
 
 // Writes the staging tile back with the remap permutation, an amplitude pair
