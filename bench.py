@@ -265,17 +265,51 @@ def pass_bounds(n, work, pass_ms, hbm_gbs, sm_mhz, nsm):
                       "smem_bytes_per_sm_clk": SMEM_BYTES_PER_SM_CLK, "sms": nsm}}
 
 
-def committed_traffic(n):
-    """Per-launch DRAM bytes of the group-pass kernel from the committed ncu
-    summary (profiles/group_pass_traffic.json), scaled to 2^n amplitudes."""
+def committed_traffic(alg_bytes):
+    """Per-launch DRAM bytes of the group-pass kernel: the DRAM bytes per
+    algorithmic byte of the committed ncu summary
+    (profiles/group_pass_traffic.json, launches that visit every coset) times
+    this run's algorithmic bytes per launch."""
     p = os.path.join(ROOT, "profiles", "group_pass_traffic.json")
     if not os.path.exists(p):
         return None
     try:
         d = json.load(open(p))
-        return d["dram_bytes_per_launch"] * (2.0 ** n) / (2.0 ** d["nqubits"])
+        return alg_bytes * d["dram_bytes_per_launch"] / d["alg_bytes_per_launch"]
     except Exception:
         return None
+
+
+def measurement_bytes(n):
+    """Device-to-host bytes of execute()'s measurement: the 2 n + 1 complex
+    amplitude sums and the error flag, which the kernels write to pinned
+    host memory."""
+    return 16 * (2 * n + 1) + 4
+
+
+def run_upload_bytes(circ, product_start):
+    """Host-to-device bytes of Simulator(circ).execute() for a complex128
+    circuit whose passes all run in specialised kernels: each pass's kernel
+    parameters (the state's address and the matrices, 16 bytes an entry; a
+    product start's first pass also the factors of 40 qubits) and the
+    workspace, whose tables such a circuit leaves empty."""
+    import ctypes
+
+    from kate_b200 import _lib
+    L = _lib.lib()
+    simulator_plan, nmats_at = 32, 12  # KATE_PLAN_SIMULATOR; PassProg::nmats
+    h, num, size, has = ctypes.c_void_p(), ctypes.c_int(), ctypes.c_size_t(), ctypes.c_int()
+    if L.kate_plan_create(circ.handle, 12, 4, simulator_plan, ctypes.byref(h)):
+        raise RuntimeError(_lib.last_error())
+    total = 1040 + (2 * 40 * 16 if product_start else 0)
+    L.kate_plan_num_passes(h, ctypes.byref(num))
+    for i in range(num.value):
+        L.kate_plan_get_program(h, i, None, 0, ctypes.byref(size), ctypes.byref(has))
+        buf = ctypes.create_string_buffer(size.value)
+        L.kate_plan_get_program(h, i, buf, size.value, ctypes.byref(size), ctypes.byref(has))
+        total += 16 + 16 * max(1, int.from_bytes(buf.raw[nmats_at:nmats_at + 4], "little"))
+    L.kate_plan_destroy(h)
+    return total
 
 
 def max_over_ranks(ms, device=None):
@@ -511,16 +545,8 @@ def main():
     e2e_ms = (time.perf_counter() - t0) * 1000.0 / e2e_steps
     if dist:
         e2e_ms = max_over_ranks(e2e_ms, dev)
-    n_ops = sum(ng for _, ng in passes)
-    h2d = n_ops * 112 + 16 * (4 ** 1) * n_ops + 2 * n * 8
-    # proba_state: per-CTA partial sums of the bit-sum kernel (2^g CTAs,
-    # 1 + 2 (12 + r) complex sums each, g = min(n - 12, 10), r = the rest up
-    # to 8), then the (theta, phi) pairs.
-    g_bits = min(n - 12, 10)
-    r_bits = n - 12 - g_bits
-    if r_bits > 8:
-        g_bits, r_bits = n - 12 - 8, 8
-    d2h = 2 * n * 8 + 16 * (1 + 2 * (12 + r_bits)) * (1 << g_bits)
+    h2d = run_upload_bytes(circ, product_start=True)
+    d2h = measurement_bytes(n)
 
     ref_gpu = None
     if rank == 0 and world == 1 and not args.no_ref_gpu:
@@ -549,7 +575,7 @@ def main():
                 "e2e": {"value": world * L / (e2e_ms / 1000.0), "unit": UNIT, "h2d_bytes_per_step": h2d,
                         "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                             "frac": achieved / peak, "traffic": committed_traffic(n),
+                             "frac": achieved / peak, "traffic": committed_traffic(alg_bytes),
                              "peak_source": peak_kind, "kernel": PASS_KERNEL,
                              "alg_bytes_per_launch": alg_bytes, "avg_launch_ms": avg_pass_ms,
                              "profiled_pass_ms": {"min": min(pass_ms), "max": max(pass_ms),
@@ -708,7 +734,7 @@ def run_precision(args):
         f"{n}q SU(4) brickwork layers/s (complex64)", "layers/s", L * 1000.0 / ms, args, ms, "c64 (split-bf16 x3 products / f32 accumulation)",
         cfg,
         e2e={"value": L * 1000.0 / e2e_ms, "unit": "layers/s", "h2d_bytes_per_step": len(gates) * 16 * 16,
-             "d2h_bytes_per_step": 2 * n * 8, "ms_per_step": e2e_ms},
+             "d2h_bytes_per_step": measurement_bytes(n), "ms_per_step": e2e_ms},
         roofline={"bound": "hbm", "achieved": alg / (avg_pass / 1000) / 1e9, "peak": peak, "unit": "GB/s",
                   "frac": alg / (avg_pass / 1000) / 1e9 / peak, "traffic": None, "peak_source": peak_kind,
                   "kernel": "k_block_c64 (tcgen05 kind::f16, split-BF16 x3)", "alg_bytes_per_launch": alg,
@@ -821,12 +847,8 @@ def run_qulacs(args):
         e.close()
     e2e_ms = (time.perf_counter() - t0) * 1000.0 / e2e_steps
     n_ops = sum(ng for _, ng in passes)
-    h2d = n_ops * 112 + 16 * 4 * n_ops
-    g_bits = min(n - 12, 10)
-    r_bits = n - 12 - g_bits
-    if r_bits > 8:
-        g_bits, r_bits = n - 12 - 8, 8
-    d2h = 2 * n * 8 + 16 * (1 + 2 * (12 + r_bits)) * (1 << g_bits)
+    h2d = run_upload_bytes(circ, product_start=False)
+    d2h = measurement_bytes(n)
 
     ref_gpu = None
     if not args.no_ref_gpu:
@@ -866,7 +888,7 @@ def run_qulacs(args):
         e2e={"value": e2e_ms, "unit": unit, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
              "ms_per_step": e2e_ms},
         roofline={"bound": "hbm", "achieved": alg / (avg_pass / 1000) / 1e9, "peak": peak, "unit": "GB/s",
-                  "frac": alg / (avg_pass / 1000) / 1e9 / peak, "traffic": committed_traffic(n),
+                  "frac": alg / (avg_pass / 1000) / 1e9 / peak, "traffic": committed_traffic(alg),
                   "peak_source": peak_kind, "kernel": PASS_KERNEL,
                   "alg_bytes_per_launch": alg, "avg_launch_ms": avg_pass,
                   "profiled_pass_ms": {"min": min(pass_ms), "max": max(pass_ms),
