@@ -255,7 +255,9 @@ KATE_API kate_status kate_sim_pass_kernel(kate_sim* s, int i, int* kind);
 /* Work per amplitude of pass i when its pass-specialised kernel (kind 2)
  * runs it: out3 = {HBM bytes read and written, FP64 instructions (DFMA,
  * DMUL, DADD as generated), shared-memory bytes stored and loaded}; with
- * 2^n amplitudes and the GPU's rates they bound the pass's time.
+ * 2^n amplitudes and the GPU's rates they bound the time of the pass when it
+ * visits every coset (as kate_sim_profile_passes runs it, and runs from a
+ * product state do; runs from |0...0> leave cosets that are still zero out).
  * KATE_EINVAL for passes on other kernels. No counterpart in the
  * reference. */
 KATE_API kate_status kate_sim_pass_work(kate_sim* s, int i, double* out3);
@@ -279,8 +281,9 @@ KATE_API kate_status kate_sim_norm2_before_renorm(kate_sim* s, double* norm2);
 #define KATE_PLAN_C64 4u        /* complex64 plan: dense 5-qubit tensor-core blocks */
 #define KATE_PLAN_NO_DENSE2 8u  /* dense two-qubit gates as shared-memory ops, not register ops */
 #define KATE_PLAN_REMAP_SEARCH 16u /* choose the qubits moved into the low bits by trying every subset
-                                      of the tile, and the gate cap per pass among 96..144 (fewest
-                                      passes): what complex128 simulators do */
+                                      of the tile, and the gate cap per pass among 96..144 (least
+                                      estimated time): what complex128 simulators of 27 qubits and more
+                                      do */
 #define KATE_PLAN_SIMULATOR 32u /* the plan a simulator of the circuit makes (a complex64 one with KATE_PLAN_C64);
                                    max_tile, coalesce and the other flags are not looked at */
 KATE_API kate_status kate_plan_create(const kate_circuit* c, int max_tile, int coalesce, unsigned flags,

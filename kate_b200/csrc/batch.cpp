@@ -399,11 +399,14 @@ std::string Batch::create(const std::vector<const Program*>& circuits, int preci
     // the first L*s/Sn large tasks, L large tasks in all.
     std::vector<int> large, small;
     for (size_t i = 0; i < np; i++) (packs[i].small ? small : large).push_back((int)i);
-    // Cosets per pass task: at most `chunk`, and a level split into at most
-    // `split` tasks: 16 when there are few circuits, so that a level spreads
-    // over several CTAs, fewer when the circuits alone keep two waves of CTAs
-    // busy (300 resident CTAs), since a task costs its operand images or
-    // tables and the dependency's round trip beside its cosets' 4.7 us each.
+    // Cosets per pass task: at most `chunk` (a level of more than `split`
+    // times that is more tasks than `split`), and below that a `split`th of
+    // the state's cosets: 16 when there are few circuits, so that a level
+    // spreads over several CTAs, fewer when the circuits alone keep two waves
+    // of CTAs busy (300 resident CTAs), since a task costs its operand images
+    // or tables and the dependency's round trip beside its cosets' 4.7 us
+    // each. Levels that visit only some of the cosets are fewer tasks of the
+    // same size.
     // With 300, 600, 900 and 1300 here 192 circuits of 10 to 20 qubits take
     // 5.10, 5.15, 5.28 and 5.45 ms, 96 of 14 to 18 1.96, 1.68, 1.85 and 1.97.
     const uint32_t split = (uint32_t)std::min<size_t>(16, std::max<size_t>(1, 600 / std::max<size_t>(1, large.size())));

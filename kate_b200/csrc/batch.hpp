@@ -29,7 +29,7 @@ struct BatchTune {
 };
 
 struct BatchOptions {
-    int chunk = 16;               // cosets per PASS task at most (and a level in at most 16 tasks)
+    int chunk = 16;               // cosets per PASS task at most (fewer where that leaves a level under 16 tasks)
     int zchunks = 4;              // 2^16-amplitude chunks per ZRED task
     uint64_t window_bytes = 0;    // queue large circuits in windows of this many state bytes (0: one window)
     std::vector<BatchTune> tune;  // by qubit count (index n); missing entries use the defaults

@@ -625,9 +625,11 @@ PlanOptions simulator_plan_options(int n, int precision) {
     // Complex128 passes of 27 qubits and more choose the qubits they move
     // into the low bits by trying every subset, and the gate cap per pass
     // among a few (about 15 ms of planning for a 30-qubit, 1780-gate
-    // circuit; below 27 qubits a pass takes under 0.7 ms and the search
-    // would cost more host time than it saves). KATE_REMAP_SEARCH=0 or 1
-    // forces it off or on.
+    // circuit). Below 27 qubits the search takes 2 to 4 ms more than a plan
+    // without it, which one run does not win back (10 layers at 24 qubits: 9
+    // passes in place of 23, about 1.2 ms less; at 26 qubits 8 in place of 18,
+    // 3.3 ms); a simulator that runs often would, from 20 qubits on (6 passes
+    // in place of 10). KATE_REMAP_SEARCH=0 or 1 forces it off or on.
     {
         const char* rs = std::getenv("KATE_REMAP_SEARCH");
         const bool on = rs ? std::atoi(rs) != 0 : n >= 27;
@@ -679,8 +681,9 @@ std::string build_plan(const Program& prog, const PlanOptions& opt, Plan* out) {
         // 30-qubit plans at each cap): 7 % off in the mean square, and in the
         // measured order for the 30-qubit plans (203, 210, 215 and 227 ps for
         // caps 144, 128, 112 and 96). Passes with shared-memory ops
-        // (interpreter) or without a register-staged program (generic
-        // kernel) count three and ten HBM passes.
+        // (dense gates of three to five qubits on the tile) or without a
+        // register-staged program (generic kernel) count three and ten HBM
+        // passes, whatever their gates; the fit has none of them.
         auto cost = [](const PlannedPass& pp) {
             const double hbm = 4.9;
             if (!pp.prog) return 10 * hbm;

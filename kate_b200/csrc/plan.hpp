@@ -27,8 +27,9 @@
 // selection reaches. The pass count then depends on the gate cap per pass
 // in no monotone way (a cap cuts a pass's gates to a program-order prefix,
 // which changes what the next pass can reach); with cap_search the planner
-// plans with each of a few caps and keeps the plan with the fewest passes
-// (passes left without a register-staged program count as ten).
+// plans with each of a few caps and keeps the plan with the least estimated
+// time (the sum over its passes of the largest of HBM, FP64 and
+// shared-memory time; plan.cpp).
 #pragma once
 
 #include <cstdint>
@@ -48,7 +49,7 @@ struct PlanOptions {
     int coalesce = 4;    // c: low physical bits every tile must contain
     bool remap = true;   // move next-needed qubits into the low bits on write
     bool remap_search = false;  // choose those qubits by trying every c-subset of the tile
-    bool cap_search = false;    // plan with several gate caps per pass, keep the plan with the fewest passes
+    bool cap_search = false;    // plan with several gate caps per pass, keep the cheapest by its estimate
     bool fuse_1q = true; // multiply chains of single-qubit ops on one qubit (FP64, host)
     bool lower_all = true;  // device ops for every pass (false: only for passes the generic kernel runs)
     bool staged = true;  // build register-staged programs for the tile kernel
